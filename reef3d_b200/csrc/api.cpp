@@ -235,7 +235,8 @@ TileArgs make_tile_args(r3d_handle* h, int stage) {
     double hmin = h->M.h[0];
     for (int d = 0; d < 3; ++d) {
         a.rh[d] = (float)(1.0 / h->M.h[d]);
-        a.eps[d] = (float)(1.0 / (h->M.h[d] * h->M.h[d]));
+        a.psi1[d] = (float)(0.3e-6 * h->M.h[d] * h->M.h[d]);
+        a.psi2[d] = (float)(0.75e-6 * h->M.h[d] * h->M.h[d]);
         const double hb = 1.0 / (double)a.rh[d];
         a.beps[d] = 1.0e-6 * hb * hb;
         hmin = std::fmin(hmin, h->M.h[d]);
@@ -488,8 +489,11 @@ int r3d_create(const r3d_grid_desc* desc, r3d_handle** out) {
     launch_set_scalar(h->S.vscale, 1.0, h->stream);
     cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return bail(R3D_EDEVICE, std::string("initialisation: ") + cudaGetErrorString(e));
-    // the tiled kernels index a field with 32-bit offsets
-    if (fp32(h) && !h->L.two_d && h->M.uniform && h->L.ncell < (1ll << 31)) {
+    // the tiled kernels index a field with 32-bit offsets, and their WENO psi
+    // (1e-6 h^2) has to be a normal FP32 number
+    bool h_ok = true;
+    for (int a = 0; a < 3; ++a) h_ok = h_ok && h->M.h[a] > 1.0e-14 && h->M.h[a] < 1.0e14;
+    if (fp32(h) && !h->L.two_d && h->M.uniform && h_ok && h->L.ncell < (1ll << 31)) {
         std::string why;
         const int ids[3] = {R3D_PHI, R3D_WORK1, R3D_WORK2};
         bool ok = true;

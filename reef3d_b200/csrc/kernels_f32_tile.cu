@@ -94,59 +94,53 @@ __device__ __forceinline__ float2 sel2(bool cx, bool cy, float2 a, float2 b) {
     return make_float2(cx ? a.x : b.x, cy ? a.y : b.y);
 }
 
-// WENO5 (Jiang-Peng) derivative times h from the undivided differences
-// d1..d5 of the minus-side upwind set; the plus side passes the mirrored
-// set (d1..d5 = D2, D1, D0, D-1, D-2).  Ideal weights 0.1/0.6/0.3 for the
-// stencils (d1,d2,d3)/(d2,d3,d4)/(d3,d4,d5).
-// The smoothness indicators are formed at the scale of divided differences
-// (IS coefficients times 1/h^2, so s = IS + psi with the reference's
-// psi = 1e-6 exactly as in src/weno_nug_func.h:133-143), and the nonlinear
-// weights w_r = (c_r/s_r^2) / sum_q (c_q/s_q^2) are evaluated with one
-// reciprocal as n_r / sum_q n_q, n_r = prod_{q!=r} t_q^2, where
-// t_q = s_q / sqrt(c_q) (the 1/sqrt(c_q) folded into the coefficients of s_q).
-// ih2 = 1/h^2 of the axis.
-__device__ __forceinline__ float2 weno5_2(float2 d1, float2 d2, float2 d3, float2 d4, float2 d5, float ih2) {
-    const float2 a1 = sub2(d3, d4), b1 = sub2(d5, d4);
-    const float2 b2 = sub2(d2, d3), b3 = sub2(d1, d2);
-    // s_r scaled by 1/sqrt(c_r) (c = 0.3, 0.6, 0.1): n_r = prod_{q!=r} s_q^2;
-    // s1 = IS1 + psi = (10/3 a1 + 11/3 b1) a1 + 4/3 b1^2 + psi,
-    // IS2 = (4/3 a1 - 5/3 b2) a1 + 4/3 b2^2, IS3 = (10/3 b2 - 11/3 b3) b2 + 4/3 b3^2
-    constexpr float G1 = 1.8257418583505538f, G2 = 1.2909944487358056f, G3 = 3.1622776601683795f;
-    const float2 s1 = fma2(fma2(f2(ih2 * (10.0f / 3.0f * G1)), a1, mul2(f2(ih2 * (11.0f / 3.0f * G1)), b1)), a1,
-                           fma2(mul2(f2(ih2 * (4.0f / 3.0f * G1)), b1), b1, f2(1.0e-6f * G1)));
-    const float2 s2 = fma2(fma2(f2(ih2 * (4.0f / 3.0f * G2)), a1, mul2(f2(ih2 * (-5.0f / 3.0f * G2)), b2)), a1,
-                           fma2(mul2(f2(ih2 * (4.0f / 3.0f * G2)), b2), b2, f2(1.0e-6f * G2)));
-    const float2 s3 = fma2(fma2(f2(ih2 * (10.0f / 3.0f * G3)), b2, mul2(f2(ih2 * (-11.0f / 3.0f * G3)), b3)), b2,
-                           fma2(mul2(f2(ih2 * (4.0f / 3.0f * G3)), b3), b3, f2(1.0e-6f * G3)));
-    // IS + psi clamped at 1e6 (fields far from a distance function): the
-    // products below stay inside the FP32 range
-    const float2 c1 = make_float2(fminf(s1.x, 1.0e6f * G1), fminf(s1.y, 1.0e6f * G1));
-    const float2 c2 = make_float2(fminf(s2.x, 1.0e6f * G2), fminf(s2.y, 1.0e6f * G2));
-    const float2 c3 = make_float2(fminf(s3.x, 1.0e6f * G3), fminf(s3.y, 1.0e6f * G3));
-    const float2 q1 = mul2(c1, c1), q2 = mul2(c2, c2), q3 = mul2(c3, c3);
-    const float2 n1 = mul2(q2, q3);
-    const float2 n2 = mul2(q1, q3);
-    const float2 n3 = mul2(q1, q2);
-    const float2 inv = rcp2(add2(add2(n1, n2), n3));
-    // p1 = d4 + a1/3 - b1/6, p2 = d3 - a1/3 - b2/6, p3 = d2 + b3/3 - 11/6 b2
-    const float2 p1 = fma2(f2(-1.0f / 6.0f), b1, fma2(f2(1.0f / 3.0f), a1, d4));
-    const float2 p2 = fma2(f2(-1.0f / 6.0f), b2, fma2(f2(-1.0f / 3.0f), a1, d3));
-    const float2 p3 = fma2(f2(-11.0f / 6.0f), b2, fma2(f2(1.0f / 3.0f), b3, d2));
-    return mul2(fma2(n3, p3, fma2(n2, p2, mul2(n1, p1))), inv);
+// WENO5 (Jiang-Peng) on a uniform axis, twice the derivative times h, as the
+// central difference M = f[+1] - f[-1] less a correction of the second
+// differences E_j = f[j+1] - 2 f[j] + f[j-1] around the cell.  With
+//   a, b, c, d = E_-2, E_-1, E_0, E_+1   (minus side; the plus side mirrors
+//   the axis: E_+2, E_+1, E_0, E_-1, and the correction changes its sign)
+// the three smoothness indicators plus psi = 1e-6, times h^2 and over their
+// leading coefficients, are sums of squares,
+//   s1 = (c - 0.55 d)^2 + 0.0975 d^2 + 0.3e-6 h^2      (IS1 10/3 of it)
+//   s2 = (b - 0.625 c)^2 + 0.609375 c^2 + 0.75e-6 h^2  (IS2  4/3 of it)
+//   s3 = (b - 0.55 a)^2 + 0.0975 a^2 + 0.3e-6 h^2      (IS3 10/3 of it)
+// and the weights w_r = (c_r/s_r^2) / sum enter through the ratios p = s1/s2,
+// q = s3/s2: with P = p^2, Q = 1.5 q^2 the correction is
+//   (1/3) [ c - b + (P (a-2b+c) + Q (b-2c+d)) / (P/2 + Q + 12.5 P Q) ].
+// Ratios need no scaling against the FP32 range whatever h is.  One of p, q
+// is always above 0.05 (s1 >= 0.24 c^2, s3 >= 0.24 b^2, s2 <= 2 (b^2 + c^2)
+// plus the psi terms), so the denominator cannot vanish; 1e-15 (s1 + s3)
+// added to s2 bounds the ratios by 1e15, so that no square of a field far
+// from a distance function leaves the FP32 range (the weight it changes is
+// below 1e-12).
+// 31 packed operations and no clamps after the selects, where the form with
+// three products of squared indicators took 37 and 6, and half the distinct
+// constants (the registers that hold them limit the CTAs per SM).  With the
+// plane loop's address and wall-ghost arithmetic cut at the same time, the
+// 256^3 stages went 140 -> 121 us (convection, 397 -> ~340 warp instructions
+// per 64 cells; issue-bound) and 187 -> 133 us (reinitialisation of five
+// spheres, most of it the interface band below).
+__device__ __forceinline__ float2 weno5_corr(float2 a, float2 b, float2 c, float2 d, float psi1, float psi2) {
+    const float2 x1 = fma2(f2(-0.55f), d, c), x2 = fma2(f2(-0.625f), c, b), x3 = fma2(f2(-0.55f), a, b);
+    const float2 s1 = fma2(x1, x1, fma2(mul2(f2(0.0975f), d), d, f2(psi1)));
+    const float2 s2 = fma2(x2, x2, fma2(mul2(f2(0.609375f), c), c, f2(psi2)));
+    const float2 s3 = fma2(x3, x3, fma2(mul2(f2(0.0975f), a), a, f2(psi1)));
+    const float2 rho = rcp2(fma2(f2(1.0e-15f), add2(s1, s3), s2));
+    const float2 p = mul2(s1, rho), q = mul2(s3, rho);
+    const float2 P = mul2(p, p), Q = mul2(mul2(f2(1.5f), q), q);
+    const float2 inv = rcp2(fma2(P, fma2(Q, f2(12.5f), f2(0.5f)), Q));
+    const float2 F = sub2(c, b);
+    const float2 G0 = add2(sub2(a, b), F), G2 = sub2(sub2(d, c), F);
+    return fma2(fma2(P, G0, mul2(Q, G2)), inv, F);
 }
 
-// Upwind derivative (times h) of an axis from its six packed undivided
-// differences D[m] = f[m+1] - f[m] of the 7-point stencil f[0..6] (f[3] the
-// cells), plus side where `plus` is set per cell.
-__device__ __forceinline__ float2 deriv2(const float2* D, bool px, bool py, float ih2) {
-    // minus: (D0..D4); plus (mirrored): (D5, D4, D3, D2, D1)
-    return weno5_2(sel2(px, py, D[5], D[0]), sel2(px, py, D[4], D[1]), sel2(px, py, D[3], D[2]),
-                   sel2(px, py, D[2], D[3]), sel2(px, py, D[1], D[4]), ih2);
-}
-
-__device__ __forceinline__ void diffs2(const float2* f, float2* D) {
-#pragma unroll
-    for (int m = 0; m < 6; ++m) D[m] = sub2(f[m + 1], f[m]);
+// Twice the upwind derivative times h of an axis from its second differences
+// e[0..4] (cells -2..+2) and the central difference m; plus side where px, py.
+__device__ __forceinline__ float2 deriv2(const float2* e, float2 m, bool px, bool py, float psi1, float psi2) {
+    const float2 r = weno5_corr(sel2(px, py, e[4], e[0]), sel2(px, py, e[3], e[1]), e[2], sel2(px, py, e[1], e[3]),
+                                psi1, psi2);
+    constexpr float third = 1.0f / 3.0f;
+    return fma2(make_float2(px ? third : -third, py ? third : -third), r, m);
 }
 
 // WENO5 (Jiang-Peng) derivative times h in FP64 from the undivided
@@ -166,40 +160,32 @@ __device__ __forceinline__ double weno5_d(double d1, double d2, double d3, doubl
     return (n1 * p1 + n2 * p2 + n3 * p3) / (n1 + n2 + n3);
 }
 
-// Reinitialisation right-hand side of one cell in FP64 from its FP32
-// stencils (the interface band): Godunov selection, one-sided WENO5 per
-// axis and the smoothed sign of src/reinidisc_f.cpp:58-127 on a uniform
-// grid.  X, Y, Z: the 7-point stencils along x, y, z (centre at [3]); rh*:
-// the FP32 1/h per axis, eps* = 1e-6 h^2 with h = 1/(double)rh (host-made).
-__device__ __noinline__ float reini_cell_fp64(const float* X, const float* Y, const float* Z, float rhx, float rhy,
-                                              float rhz, double epsx, double epsy, double epsz, float deltax) {
-    const float rh[3] = {rhx, rhy, rhz};
-    const double epsd[3] = {epsx, epsy, epsz};
-    const double f0 = X[3];
-    const double sg = fabs(f0) < 1.0e-8 ? 1.0 : (f0 > 0.0 ? 1.0 : -1.0);
-    const float* ax[3] = {X, Y, Z};
-    double g2 = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const float* f = ax[d];
-        double D[6];
-#pragma unroll
-        for (int m = 0; m < 6; ++m) D[m] = (double)f[m + 1] - (double)f[m];
-        const double ms = D[2] * sg, ps = D[3] * sg, sum = ms + ps;
-        const bool c1 = ms > 0.0 && sum > 0.0, c2 = ps < 0.0 && sum < 0.0;
-        if (c1 || c2) {
-            const double eps = epsd[d];
-            const double w = c2 ? weno5_d(D[5], D[4], D[3], D[2], D[1], eps)
-                                : weno5_d(D[0], D[1], D[2], D[3], D[4], eps);
-            const double gd = w * (double)rh[d];
-            g2 += gd * gd;
-        }
-    }
+// The interface band of the reinitialisation in FP64: the Godunov selection
+// and one-sided WENO5 of one axis (src/reinidisc_f.cpp:70-109 on a uniform
+// grid), squared, from the FP32 7-point stencil of the axis (centre f3): rh
+// the FP32 1/h, eps = 1e-6 h^2 with h = 1/(double)rh (host-made).
+__device__ __noinline__ double band_axis(float f0, float f1, float f2_, float f3, float f4, float f5, float f6,
+                                         float rh, double eps) {
+    const double sg = fabs((double)f3) < 1.0e-8 ? 1.0 : (f3 > 0.f ? 1.0 : -1.0);
+    const double D2 = (double)f3 - (double)f2_, D3 = (double)f4 - (double)f3;
+    const double ms = D2 * sg, ps = D3 * sg, sum = ms + ps;
+    const bool c1 = ms > 0.0 && sum > 0.0, c2 = ps < 0.0 && sum < 0.0;
+    if (!(c1 || c2)) return 0.0;
+    const double D0 = (double)f1 - (double)f0, D1 = (double)f2_ - (double)f1;
+    const double D4 = (double)f5 - (double)f4, D5 = (double)f6 - (double)f5;
+    const double w = weno5_d(c2 ? D5 : D0, c2 ? D4 : D1, c2 ? D3 : D2, c2 ? D2 : D3, c2 ? D1 : D4, eps);
+    const double gd = w * (double)rh;
+    return gd * gd;
+}
+
+// The right-hand side -(S |grad| - S) of a band cell of value f0 from the
+// squared gradient, with the smoothed sign of src/reinidisc_f.cpp:111-127.
+__device__ __forceinline__ float band_rhs(float f0f, double g2, float deltax) {
+    const double f0 = f0f, dl = deltax;
     const double dn = sqrt(g2);
-    const double dl = deltax;
-    double S = f0 / sqrt(f0 * f0 + dn * dn * dl * dl);
+    double S = f0 * rsqrt(f0 * f0 + g2 * dl * dl);
     if (S != S) S = 1.0;
-    return (float)(S - S * dn);  // -(S |grad| - S)
+    return (float)(S - S * dn);
 }
 
 // Position of the n-th (from 0) set bit of m, for n < popc(m): a binary
@@ -252,6 +238,7 @@ struct TileCfg {
 };
 
 // The configurations the library is built with (id = position).
+#ifndef R3D_TILE_CFGS
 #define R3D_TILE_CFGS(X)        \
     X(0, 64, 8, 1, 16, 3)       \
     X(1, 64, 8, 2, 12, 4)       \
@@ -260,6 +247,7 @@ struct TileCfg {
     X(4, 128, 8, 2, 8, 2)       \
     X(5, 64, 8, 1, 10, 4)       \
     X(6, 32, 16, 2, 12, 5)
+#endif
 
 #define R3D_CFG_TYPE(id, tx, ty, ry, ring, minb) using Cfg##id = TileCfg<tx, ty, ry, ring, minb>;
 R3D_TILE_CFGS(R3D_CFG_TYPE)
@@ -282,7 +270,7 @@ R3D_TILE_CFGS(R3D_CFG_TYPE)
 // release counter), so that warps drift apart where their work differs
 // (interface-band cells in FP64, wall ghosts) instead of meeting at a CTA
 // barrier every plane.
-template <class C, bool REINI, int STAGE, bool ISO>
+template <class C, bool REINI, int STAGE, bool ISO, bool REUSE>
 __device__ __forceinline__ bool tile_item(const CUtensorMap* tmap, const TileArgs& a, int bx, int by, int bz,
                                           bool volume, unsigned char* smem_raw, double* red_a, double* red_b,
                                           double* partial_out) {
@@ -305,25 +293,29 @@ __device__ __forceinline__ bool tile_item(const CUtensorMap* tmap, const TileArg
     const int ybox = by * C::TY + L.gy - 3;
     const int pfirst = k0 - 3;  // first plane staged (ring position 0)
     const int plast = k1 + 2;   // last plane staged
-    const int rowb = tg * RY;   // box row of the first y-stencil point of the thread's first row
-    bool act0[RY], act1[RY], gside[RY], gxlo[RY], gxhi1[RY], gxhi2[RY], gylo[RY], gyhi[RY];
-    int col[RY];  // 32-bit offsets: the host enables tiles only for fields of < 2^31 cells
-    int own[RY];  // the thread's two cells of row r in a box
+    const int own = (tg * RY + 3) * BX + 2 * tx + 4;  // the thread's first two cells in a box
+    // The thread's cells within a plane, as unsigned offsets from the plane's
+    // (CTA-uniform) base pointers, so a load or store costs no 64-bit address
+    // arithmetic per thread.  Loads are unconditional: a thread outside the
+    // grid reads the nearest cell pair of its rows instead (the pair after
+    // the last cell ends in the ghost layer), and its values go nowhere.
+    const unsigned col0 = (unsigned)((jb + L.gy) * sy + (i0 + L.gx));
+    unsigned ld[RY];
+    // bits per row r (shifted by 8 r): 1 first cell inside, 2 second cell
+    // inside, 4 x-min wall, 8 x-max wall (second cell), 16 x-max wall (first
+    // cell), 32 y-min wall, 64 y-max wall
+    unsigned flags = 0;
 #pragma unroll
     for (int r = 0; r < RY; ++r) {
         const int j = jb + r;
-        act0[r] = i0 < L.nx && j < L.ny;
-        act1[r] = i0 + 1 < L.nx && j < L.ny;
-        col[r] = (j + L.gy) * sy + (i0 + L.gx);
-        own[r] = (rowb + r + 3) * BX + 2 * tx + 4;
-        // wall ghost layers this thread writes on every plane (x, y faces)
-        gxlo[r] = act0[r] && i0 == 0;
-        gxhi2[r] = act1[r] && i0 + 1 == L.nx - 1;  // second cell is the last one
-        gxhi1[r] = act0[r] && !act1[r];             // first cell is the last one
-        gylo[r] = act0[r] && j == 0;
-        gyhi[r] = act0[r] && j == L.ny - 1;
-        gside[r] = gxlo[r] || gxhi2[r] || gxhi1[r] || gylo[r] || gyhi[r];
+        ld[r] = (unsigned)((min(j, L.ny - 1) + L.gy) * sy + (min(i0, (L.nx - 1) & ~1) + L.gx));
+        const bool in0 = i0 < L.nx && j < L.ny, in1 = i0 + 1 < L.nx && j < L.ny;
+        const unsigned f = (in0 ? 1u : 0u) | (in1 ? 2u : 0u) | (in0 && i0 == 0 ? 4u : 0u) |
+                           (in1 && i0 + 1 == L.nx - 1 ? 8u : 0u) | (in0 && !in1 ? 16u : 0u) |
+                           (in0 && j == 0 ? 32u : 0u) | (in0 && j == L.ny - 1 ? 64u : 0u);
+        flags |= f << (8 * r);
     }
+    const unsigned ldm = (unsigned)((min(jb, L.ny - 1) + L.gy - 1) * sy + (min(i0, (L.nx - 1) & ~1) + L.gx));
 
     if (tid == 0) {
         for (int s = 0; s < RING; ++s) {
@@ -349,21 +341,17 @@ __device__ __forceinline__ bool tile_item(const CUtensorMap* tmap, const TileArg
     // timeout-path test: the second completion of box 0 needs a refill that
     // only the plane loop issues, so this wait gives up after `spin` tries
     if (a.wait_test) ok = ok && mbar_wait_bounded(bar, 1, spin);
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) *s_abort = 1;
 
     const float vs = (float)*a.vscale;
     const float dtc = REINI ? a.dtr : (float)*a.dt;
-    const int c0 = (k0 + L.gz) * sz;
+    // plane base pointers, advanced with k
+    const size_t c0 = (size_t)(k0 + L.gz) * (size_t)L.sz;
+    const float *pu = a.u + c0, *pv = a.v + c0, *pw = a.w + c0, *pf = a.fn + c0;
+    float* po = a.out + c0;
     float2 wprev[RY];
 #pragma unroll
-    for (int r = 0; r < RY; ++r) {
-        wprev[r] = make_float2(0.f, 0.f);
-        if (!REINI && act0[r]) {
-            const float* wp = a.w + c0 + col[r] - sz;
-            wprev[r] = act1[r] ? __ldg(reinterpret_cast<const float2*>(wp)) : make_float2(__ldg(wp), 0.f);
-        }
-    }
+    for (int r = 0; r < RY; ++r)
+        if (!REINI) wprev[r] = __ldg(reinterpret_cast<const float2*>(pw - sz + ld[r]));
     double vol_a = 0.0, vol_b = 0.0;
 
     // cell-local global operands of a plane (velocities, step start value),
@@ -371,83 +359,85 @@ __device__ __forceinline__ bool tile_item(const CUtensorMap* tmap, const TileArg
     // v on the face below row r is v of row r-1 for r > 0
     float2 nu[RY], nv[RY], nw[RY], nfn[RY], nvm0;
     float num[RY];
-#pragma unroll
-    for (int r = 0; r < RY; ++r) {
-        nu[r] = nv[r] = nw[r] = nfn[r] = make_float2(0.f, 0.f);
-        num[r] = 0.f;
-    }
-    nvm0 = make_float2(0.f, 0.f);
-    auto fetch = [&](int cz) {
+    auto fetch = [&]() {
 #pragma unroll
         for (int r = 0; r < RY; ++r) {
-            if (!act0[r]) continue;
-            const int cc = cz + col[r];
             if (!REINI) {
-                if (act1[r]) {
-                    nu[r] = __ldg(reinterpret_cast<const float2*>(a.u + cc));
-                    nv[r] = __ldg(reinterpret_cast<const float2*>(a.v + cc));
-                    nw[r] = __ldg(reinterpret_cast<const float2*>(a.w + cc));
-                    if (r == 0) nvm0 = __ldg(reinterpret_cast<const float2*>(a.v + cc - sy));
-                } else {
-                    nu[r].x = __ldg(a.u + cc);
-                    nv[r].x = __ldg(a.v + cc);
-                    nw[r].x = __ldg(a.w + cc);
-                    if (r == 0) nvm0.x = __ldg(a.v + cc - sy);
-                }
-                num[r] = __ldg(a.u + cc - 1);
+                nu[r] = __ldg(reinterpret_cast<const float2*>(pu + ld[r]));
+                num[r] = __ldg(pu + ld[r] - 1);
+                nv[r] = __ldg(reinterpret_cast<const float2*>(pv + ld[r]));
+                nw[r] = __ldg(reinterpret_cast<const float2*>(pw + ld[r]));
             }
-            // the step start value may be this stage's output (stage 3): plain loads
-            if (STAGE != 1) nfn[r] = act1[r] ? *reinterpret_cast<const float2*>(a.fn + cc) : make_float2(a.fn[cc], 0.f);
+            // the step start value may be this stage's output (stage 3): plain
+            // loads, and of the thread's own cells alone
+            if (STAGE == 2 || (STAGE == 3 && ((flags >> (8 * r)) & 1u))) nfn[r] = *reinterpret_cast<const float2*>(pf + ld[r]);
         }
+        if (!REINI) nvm0 = __ldg(reinterpret_cast<const float2*>(pv + ldm));
+        pu += sz;
+        pv += sz;
+        pw += sz;
+        pf += sz;
     };
-    fetch(c0);
+    fetch();
 
+    constexpr int AY = ISO ? 0 : 1, AZ = ISO ? 0 : 2;
+    int z[7];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) z[m + 1] = m * SLOT + own;
     int sb = 0;          // ring slot of position n = k - k0 (plane k-3)
     int ws = 6, wp = 0;  // ring slot and phase parity of position n + 6 (plane k+3)
-    int cz = c0;
-    for (int k = k0; k < k1; ++k, cz += sz) {
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar + ws, (uint32_t)wp, spin));
-        if (!ok) *s_abort = 1;
-        if (__any_sync(0xffffffffu, *s_abort != 0)) break;
-        const float* slot[7];
-#pragma unroll
-        for (int m = 0; m < 7; ++m) {
-            int s = sb + m;
-            if (RING < 16 || (RING & (RING - 1))) s -= s >= RING ? RING : 0;
-            else s &= RING - 1;
-            slot[m] = ring + s * SLOT;
+    for (int k = k0; k < k1; ++k, po += sz) {
+        ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(bar + ws, (uint32_t)wp, spin));
+        // a warp whose wait gave up leaves; the boxes it no longer releases
+        // are not refilled, so the other warps' waits give up in turn
+        if (!ok) {
+            *s_abort = 1;
+            break;
         }
-        const float* sl = slot[3];  // plane k
+        // the thread's own column in the boxes of planes k-3 .. k+3 (ring
+        // offsets), moved on by one plane
+#pragma unroll
+        for (int m = 0; m < 6; ++m) z[m] = z[m + 1];
+        z[6] = ws * SLOT + own;
+        const float* zc[7];
+#pragma unroll
+        for (int m = 0; m < 7; ++m) zc[m] = ring + z[m];
+        const float* sl = zc[3];
 
-        // y stencil values of all RY rows (rows rowb .. rowb+RY+5 of the box)
-        float2 DY[RY + 5];
+        // y stencil values of all RY rows, first and second differences
+        float2 DY[RY + 5], EY[RY + 4], MY[RY];
         float2 fy2[RY], fy4[RY];
         {
             float2 fy[RY + 6];
 #pragma unroll
-            for (int m = 0; m < RY + 6; ++m) fy[m] = *reinterpret_cast<const float2*>(sl + (rowb + m) * BX + 2 * tx + 4);
+            for (int m = 0; m < RY + 6; ++m) fy[m] = *reinterpret_cast<const float2*>(sl + (m - 3) * BX);
 #pragma unroll
             for (int m = 0; m < RY + 5; ++m) DY[m] = sub2(fy[m + 1], fy[m]);
 #pragma unroll
-            for (int r = 0; r < RY; ++r) { fy2[r] = fy[r + 2]; fy4[r] = fy[r + 4]; }
+            for (int m = 0; m < RY + 4; ++m) EY[m] = sub2(DY[m + 1], DY[m]);
+#pragma unroll
+            for (int r = 0; r < RY; ++r) { fy2[r] = fy[r + 2]; fy4[r] = fy[r + 4]; MY[r] = sub2(fy4[r], fy2[r]); }
         }
         // this plane's operands, then the next plane's loads in flight
         // through the whole computation of this one
         float2 fnr[RY], ucr[RY], vcr[RY], wcr[RY], vm0;
         float umr[RY];
 #pragma unroll
-        for (int r = 0; r < RY; ++r) { fnr[r] = nfn[r]; ucr[r] = nu[r]; vcr[r] = nv[r]; wcr[r] = nw[r]; umr[r] = num[r]; }
-        vm0 = nvm0;
-        if (k + 1 < k1) fetch(cz + sz);
+        for (int r = 0; r < RY; ++r) {
+            if (STAGE != 1) fnr[r] = nfn[r];
+            if (!REINI) { ucr[r] = nu[r]; vcr[r] = nv[r]; wcr[r] = nw[r]; umr[r] = num[r]; }
+        }
+        if (!REINI) vm0 = nvm0;
+        if (k + 1 < k1) fetch();
 
         float2 f0[RY], Lc[RY];
         bool bandx[RY], bandy[RY];
 #pragma unroll
         for (int r = 0; r < RY; ++r) {
             // x stencil: the row's columns 2tx .. 2tx+9 (the cells at 2tx+4, 2tx+5)
-            float xv[10];
+            float xv[10], dx[9], ex[8];
             {
-                const float* rp = sl + (rowb + r + 3) * BX + 2 * tx;
+                const float* rp = sl + r * BX - 4;
 #pragma unroll
                 for (int q = 0; q < 5; ++q) {
                     const float2 t = *reinterpret_cast<const float2*>(rp + 2 * q);
@@ -455,65 +445,77 @@ __device__ __forceinline__ bool tile_item(const CUtensorMap* tmap, const TileArg
                     xv[2 * q + 1] = t.y;
                 }
             }
-            float2 Dx[6], Dz[6];
 #pragma unroll
-            for (int m = 0; m < 6; ++m) Dx[m] = make_float2(xv[m + 2] - xv[m + 1], xv[m + 3] - xv[m + 2]);
-            float2 fz2, fz4;
+            for (int m = 1; m < 8; ++m) dx[m] = xv[m + 1] - xv[m];
+#pragma unroll
+            for (int m = 2; m < 8; ++m) ex[m] = dx[m] - dx[m - 1];  // about column m
+            float2 DZ[6], EZ[5], fz2, fz4;
             {
                 float2 fz[7];
 #pragma unroll
-                for (int m = 0; m < 7; ++m) fz[m] = *reinterpret_cast<const float2*>(slot[m] + own[r]);
-                diffs2(fz, Dz);
+                for (int m = 0; m < 7; ++m) fz[m] = *reinterpret_cast<const float2*>(zc[m] + r * BX);
+#pragma unroll
+                for (int m = 0; m < 6; ++m) DZ[m] = sub2(fz[m + 1], fz[m]);
+#pragma unroll
+                for (int m = 0; m < 5; ++m) EZ[m] = sub2(DZ[m + 1], DZ[m]);
                 fz2 = fz[2];
                 fz4 = fz[4];
             }
-            const float2* Dy = DY + r;
             f0[r] = make_float2(xv[4], xv[5]);
+            const float2 mx = make_float2(xv[5] - xv[3], xv[6] - xv[4]), mz = sub2(fz4, fz2);
+            const float2 EX[5] = {make_float2(ex[2], ex[3]), make_float2(ex[3], ex[4]), make_float2(ex[4], ex[5]),
+                                  make_float2(ex[5], ex[6]), make_float2(ex[6], ex[7])};
             bandx[r] = bandy[r] = false;
             if (!REINI) {
-                const float2 h2 = f2(0.5f * vs);
+                // the derivatives come out as 2 h times themselves
                 const float2 vm = r == 0 ? vm0 : vcr[r - 1];
-                const float2 ia = mul2(h2, add2(make_float2(umr[r], ucr[r].x), ucr[r]));
-                const float2 ja = mul2(h2, add2(vcr[r], vm));
-                const float2 ka = mul2(h2, add2(wcr[r], wprev[r]));
+                const float qv = 0.25f * vs;
+                const float2 ia = mul2(f2(qv * a.rh[0]), add2(make_float2(umr[r], ucr[r].x), ucr[r]));
+                const float2 ja = mul2(f2(qv * a.rh[AY]), add2(vcr[r], vm));
+                const float2 ka = mul2(f2(qv * a.rh[AZ]), add2(wcr[r], wprev[r]));
                 wprev[r] = wcr[r];
-                const float2 gx = mul2(f2(a.rh[0]), deriv2(Dx, ia.x < 0.f, ia.y < 0.f, a.eps[0]));
-                constexpr int AY = ISO ? 0 : 1, AZ = ISO ? 0 : 2;
-                const float2 gy = mul2(f2(a.rh[AY]), deriv2(Dy, ja.x < 0.f, ja.y < 0.f, a.eps[AY]));
-                const float2 gz = mul2(f2(a.rh[AZ]), deriv2(Dz, ka.x < 0.f, ka.y < 0.f, a.eps[AZ]));
-                Lc[r] = mul2(f2(-1.f), fma2(ka, gz, fma2(ja, gy, mul2(ia, gx))));
+                const float2 gx = deriv2(EX, mx, ia.x < 0.f, ia.y < 0.f, a.psi1[0], a.psi2[0]);
+                const float2 gy = deriv2(EY + r, MY[r], ja.x < 0.f,
+                                         ja.y < 0.f, a.psi1[AY], a.psi2[AY]);
+                const float2 gz = deriv2(EZ, mz, ka.x < 0.f, ka.y < 0.f, a.psi1[AZ],
+                                         a.psi2[AZ]);
+                Lc[r] = fma2(ka, gz, fma2(ja, gy, mul2(ia, gx)));  // -L
             } else {
                 // Godunov selection per axis (src/reinidisc_f.cpp:70-109) on the
-                // backward and forward differences D[2], D[3] times the sign s
-                // (the grid factor 1/h > 0 leaves every test unchanged):
-                //   upwind minus side: m > 0 && p > -m, i.e. m > 0 && m + p > 0
-                //   upwind plus side:  p < 0 && m < -p, i.e. p < 0 && m + p < 0
-                // (the sign of a rounded sum is the sign of the exact sum)
+                // backward and forward differences m, p, with s the sign of
+                // the cell:
+                //   minus side: s m > 0 and s (m + p) > 0,
+                //   plus side:  s p < 0 and s (m + p) < 0, else 0.
+                // m + p is the central difference M: the plus side where
+                // s M < 0, and the side's own difference has to have M's sign.
                 const float2 fc = f0[r];
-                const float2 sg = make_float2(fabsf(fc.x) < 1.0e-8f ? 1.f : (fc.x > 0.f ? 1.f : -1.f),
-                                              fabsf(fc.y) < 1.0e-8f ? 1.f : (fc.y > 0.f ? 1.f : -1.f));
-                const float2* ax[3] = {Dx, Dy, Dz};
+                const float2 sg = make_float2(fc.x > -1.0e-8f ? 1.f : -1.f, fc.y > -1.0e-8f ? 1.f : -1.f);
                 float2 g2 = make_float2(0.f, 0.f);
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
-                    const float2* D = ax[d];
-                    const float2 ms = mul2(D[2], sg), ps = mul2(D[3], sg);
-                    const float2 sum = add2(ms, ps);
-                    const bool c1x = ms.x > 0.f && sum.x > 0.f, c2x = ps.x < 0.f && sum.x < 0.f;
-                    const bool c1y = ms.y > 0.f && sum.y > 0.f, c2y = ps.y < 0.f && sum.y < 0.f;
+                    const float2 dm = d == 0 ? make_float2(dx[3], dx[4]) : d == 1 ? DY[r + 2] : DZ[2];
+                    const float2 dp = d == 0 ? make_float2(dx[4], dx[5]) : d == 1 ? DY[r + 3] : DZ[3];
+                    const float2 M = d == 0 ? mx : d == 1 ? MY[r] : mz;
+                    const float2 sM = mul2(M, sg);
+                    const bool px = sM.x < 0.f, py = sM.y < 0.f;
+                    const float2 side = mul2(sel2(px, py, dp, dm), M);
                     const int ad = ISO ? 0 : d;
-                    float2 g = mul2(f2(a.rh[ad]), deriv2(D, c2x, c2y, a.eps[ad]));
-                    g.x = (c1x || c2x) ? g.x : 0.f;
-                    g.y = (c1y || c2y) ? g.y : 0.f;
+                    float2 g = deriv2(d == 0 ? EX : d == 1 ? EY + r : EZ, M, px, py, a.psi1[ad], a.psi2[ad]);
+                    if (!ISO) g = mul2(f2(a.rh[d]), g);
+                    g.x = side.x > 0.f ? g.x : 0.f;
+                    g.y = side.y > 0.f ? g.y : 0.f;
                     g2 = fma2(g, g, g2);
                 }
+                // the derivatives came out doubled (ISO: and times h)
+                const float sc = ISO ? 0.25f * a.rh[0] * a.rh[0] : 0.25f;
+                g2 = mul2(f2(sc), g2);
                 const float2 dn = make_float2(sqrt_approx(g2.x), sqrt_approx(g2.y));
                 const float2 dl = f2(a.deltax);
                 const float2 den = fma2(mul2(mul2(dn, dn), dl), dl, mul2(fc, fc));
                 float2 S = mul2(fc, make_float2(rsqrtf(den.x), rsqrtf(den.y)));
                 if (S.x != S.x) S.x = 1.f;
                 if (S.y != S.y) S.y = 1.f;
-                Lc[r] = sub2(S, mul2(S, dn));  // -(S |grad| - S)
+                Lc[r] = sub2(mul2(S, dn), S);  // -L = S |grad| - S
                 // interface band: the 7-point stencil changes sign, i.e. neither
                 // all values >= 0 (min >= 0) nor all < 0 (max < 0)
                 const float lox = min3f(min3f(fc.x, xv[3], xv[5]), min3f(fy2[r].x, fy4[r].x, fz2.x), fz4.x);
@@ -522,55 +524,87 @@ __device__ __forceinline__ bool tile_item(const CUtensorMap* tmap, const TileArg
                 const float hiy = max3f(max3f(fc.y, xv[4], xv[6]), max3f(fy2[r].y, fy4[r].y, fz2.y), fz4.y);
                 bandx[r] = lox < 0.f && hix >= 0.f;
                 bandy[r] = loy < 0.f && hiy >= 0.f;
-                if (a.f49 == 0) {
-                    if (bandx[r]) Lc[r].x = 0.f;  // src/reinidisc_fsf.cpp:70-72
-                    if (bandy[r]) Lc[r].y = 0.f;
-                }
             }
         }
         bool band_here = false;
-        if (REINI && a.f49 != 0 && a.band64) {
 #pragma unroll
-            for (int r = 0; r < RY; ++r) band_here = band_here || (act0[r] && bandx[r]) || (act1[r] && bandy[r]);
-        }
+        for (int r = 0; r < RY; ++r) band_here = band_here || bandx[r] || bandy[r];
         // one vote for the plane: most warps hold no band cell in it
-        if (REINI && a.f49 != 0 && a.band64 && __any_sync(0xffffffffu, band_here)) {
-            // The warp's band cells of row r (at most 64) are dealt out to
-            // its lanes, one FP64 evaluation each, stencils from shared
-            // memory; results go back to the owning lanes by shuffles.
+        if (REINI && __any_sync(0xffffffffu, band_here)) {
+            if (a.f49 == 0) {
 #pragma unroll
-            for (int r = 0; r < RY; ++r) {
-                const unsigned mx = __ballot_sync(0xffffffffu, act0[r] && bandx[r]);
-                const unsigned my = __ballot_sync(0xffffffffu, act1[r] && bandy[r]);
-                if (mx | my) {
-                    const int cx = __popc(mx), total = cx + __popc(my);
-                    const unsigned below = (1u << lane) - 1u;
-                    const int bxi = __popc(mx & below), byi = cx + __popc(my & below);
-                    for (int base = 0; base < total; base += 32) {
-                        float res = 0.f;
-                        const int b = base + lane;
-                        if (b < total) {
-                            const bool isy = b >= cx;
-                            // the lane holding the (b or b-cx)-th set bit of the mask
-                            const int src = nth_set_bit(isy ? my : mx, isy ? b - cx : b);
-                            const int st = (tid & ~31) + src;  // the source lane's thread
-                            const int sx = 2 * (st % C::TPR) + (isy ? 1 : 0);
-                            const int srow = (st / C::TPR) * RY + r;  // its y-stencil base row
-                            float X[7], Y[7], Z[7];
+                for (int r = 0; r < RY; ++r) {
+                    if (bandx[r]) Lc[r].x = 0.f;  // src/reinidisc_fsf.cpp:70-72
+                    if (bandy[r]) Lc[r].y = 0.f;
+                }
+            } else if (a.band64) {
+                // The band cells of the warp's RY rows are dealt out to its
+                // lanes, stencils from shared memory, results back to the owning
+                // lanes by shuffles.  A round takes ten cells with one axis per
+                // lane, or (more than twenty left) 32 cells with all three: an
+                // FP64 WENO evaluation is a chain of ~600 cycles, so a curved
+                // interface, which leaves a few cells per row, is served in one
+                // such latency instead of three.
+                unsigned mk[2 * RY];
+                int end[2 * RY];  // cells of the masks up to and including this one
+                int total = 0;
+#pragma unroll
+                for (int q = 0; q < 2 * RY; ++q) {
+                    mk[q] = __ballot_sync(0xffffffffu, q & 1 ? (flags >> (8 * (q >> 1)) & 2u) && bandy[q >> 1]
+                                                          : (flags >> (8 * (q >> 1)) & 1u) && bandx[q >> 1]);
+                    total += __popc(mk[q]);
+                    end[q] = total;
+                }
+                const unsigned below = (1u << lane) - 1u;
+                for (int base = 0; base < total;) {
+                    const bool wide = total - base > 20;
+                    const int cells = wide ? 32 : 10;
+                    const int b = base + (wide ? lane : lane / 3);
+                    double g2 = 0.0;
+                    float fcen = 0.f, res = 0.f;
+                    if (b < total && (wide || lane < 30)) {
+                        int q = 0;
+#pragma unroll
+                        for (int m = 0; m + 1 < 2 * RY; ++m) q += b >= end[m];
+                        unsigned mq = mk[0];
+                        int first = 0;
+#pragma unroll
+                        for (int m = 1; m < 2 * RY; ++m)
+                            if (q == m) {
+                                mq = mk[m];
+                                first = end[m - 1];
+                            }
+                        const int st = (tid & ~31) + nth_set_bit(mq, b - first);  // the thread that owns the cell
+                        const int oc = ((st / C::TPR) * RY + (q >> 1) + 3) * BX + 2 * (st % C::TPR) + 4 + (q & 1);
+                        const float* cen = sl - own + oc;
+                        fcen = *cen;
+                        const int ax0 = wide ? 0 : lane - 3 * (lane / 3), ax1 = wide ? 3 : ax0 + 1;
+                        for (int ax = ax0; ax < ax1; ++ax) {
+                            float f[7];
 #pragma unroll
                             for (int m = 0; m < 7; ++m) {
-                                X[m] = sl[(srow + 3) * BX + sx + 1 + m];
-                                Y[m] = sl[(srow + m) * BX + sx + 4];
-                                Z[m] = slot[m][(srow + 3) * BX + sx + 4];
+                                const float* pz = zc[m] - own + oc;
+                                f[m] = ax == 2 ? *pz : cen[(m - 3) * (ax == 0 ? 1 : BX)];
                             }
-                            res = reini_cell_fp64(X, Y, Z, a.rh[0], a.rh[1], a.rh[2], a.beps[0], a.beps[1],
-                                                  a.beps[2], a.deltax);
+                            g2 += band_axis(f[0], f[1], f[2], f[3], f[4], f[5], f[6], ax == 0 ? a.rh[0] : ax == 1 ? a.rh[1] : a.rh[2],
+                                            ax == 0 ? a.beps[0] : ax == 1 ? a.beps[1] : a.beps[2]);
                         }
-                        const float rx = __shfl_sync(0xffffffffu, res, (bxi - base) & 31);
-                        const float ry = __shfl_sync(0xffffffffu, res, (byi - base) & 31);
-                        if (act0[r] && bandx[r] && bxi >= base && bxi < base + 32) Lc[r].x = rx;
-                        if (act1[r] && bandy[r] && byi >= base && byi < base + 32) Lc[r].y = ry;
                     }
+                    if (!wide) {
+                        const double gy = __shfl_down_sync(0xffffffffu, g2, 1), gz = __shfl_down_sync(0xffffffffu, g2, 2);
+                        g2 = (g2 + gy) + gz;
+                    }
+                    if (b < total) res = -band_rhs(fcen, g2, a.deltax);
+#pragma unroll
+                    for (int q = 0; q < 2 * RY; ++q) {
+                        const int mine = (q ? end[q - 1] : 0) + __popc(mk[q] & below) - base;
+                        const float v = __shfl_sync(0xffffffffu, res, (wide ? mine : 3 * mine) & 31);
+                        if (((mk[q] >> lane) & 1u) && mine >= 0 && mine < cells) {
+                            if (q & 1) Lc[q >> 1].y = v;
+                            else Lc[q >> 1].x = v;
+                        }
+                    }
+                    base += cells;
                 }
             }
         }
@@ -596,43 +630,56 @@ __device__ __forceinline__ bool tile_item(const CUtensorMap* tmap, const TileArg
 
 #pragma unroll
         for (int r = 0; r < RY; ++r) {
-            if (!act0[r]) continue;
             // RK combine (src/levelset_RK3.cpp:121-156, src/reini_RK3.cpp:118-135)
             float2 val;
-            const float2 sdl = fma2(f2(dtc), Lc[r], f0[r]);  // stage input + dt L
+            const float2 sdl = fma2(f2(-dtc), Lc[r], f0[r]);  // stage input + dt L
             if (STAGE == 1) {
                 val = sdl;
             } else {
                 if (STAGE == 2) val = fma2(f2(0.75f), fnr[r], mul2(f2(0.25f), sdl));
                 else val = fma2(f2(1.0f / 3.0f), fnr[r], mul2(f2(2.0f / 3.0f), sdl));
             }
-            const int c = cz + col[r];
-            if (act1[r]) *reinterpret_cast<float2*>(a.out + c) = val;
-            else a.out[c] = val.x;
+            const unsigned fl = flags >> (8 * r);
+            float* o = po + (col0 + (unsigned)(r * sy));
+            if (fl & 2u) *reinterpret_cast<float2*>(o) = val;
+            else if (fl & 1u) *o = val.x;
             // wall ghost copies (src/gc_neumann.cpp:29-54)
-            if (gside[r] || k == 0 || k == L.nz - 1) {
-                if (gxlo[r]) { a.out[c - 1] = val.x; a.out[c - 2] = val.x; a.out[c - 3] = val.x; }
-                if (gxhi2[r]) { a.out[c + 2] = val.y; a.out[c + 3] = val.y; a.out[c + 4] = val.y; }
-                if (gxhi1[r]) { a.out[c + 1] = val.x; a.out[c + 2] = val.x; a.out[c + 3] = val.x; }
-                const int nw = act1[r] ? 2 : 1;
-                if (gylo[r])
-                    for (int q = 1; q <= 3; ++q)
-                        for (int e = 0; e < nw; ++e) a.out[c - q * sy + e] = e ? val.y : val.x;
-                if (gyhi[r])
-                    for (int q = 1; q <= 3; ++q)
-                        for (int e = 0; e < nw; ++e) a.out[c + q * sy + e] = e ? val.y : val.x;
-                if (k == 0 && !(L.io & kHaloZLo))  // a slab face's ghosts come from the neighbour
-                    for (int q = 1; q <= 3; ++q)
-                        for (int e = 0; e < nw; ++e) a.out[c - q * sz + e] = e ? val.y : val.x;
-                if (k == L.nz - 1 && !(L.io & kHaloZHi))
-                    for (int q = 1; q <= 3; ++q)
-                        for (int e = 0; e < nw; ++e) a.out[c + q * sz + e] = e ? val.y : val.x;
+            if (fl & 0x1cu) {
+                // x-min: three ghosts and the padding slot before them, 16-byte aligned
+                if (fl & 4u) *reinterpret_cast<float4*>(o - 4) = make_float4(val.x, val.x, val.x, val.x);
+                if (fl & 8u) {
+                    *reinterpret_cast<float2*>(o + 2) = make_float2(val.y, val.y);
+                    o[4] = val.y;
+                }
+                if (fl & 16u) { o[1] = val.x; o[2] = val.x; o[3] = val.x; }
+            }
+            if (fl & 0x60u) {
+                // ny >= 2 here (ny = 1 is a 2D grid), so never both y walls
+                const int dir = fl & 32u ? -sy : sy;
+#pragma unroll
+                for (int q = 1; q <= 3; ++q) {
+                    o[q * dir] = val.x;
+                    if (fl & 2u) o[q * dir + 1] = val.y;
+                }
+            }
+            if (k == 0 || k == L.nz - 1) {
+                // a slab face's ghosts come from the neighbour
+                if (k == 0 && !(L.io & kHaloZLo) && (fl & 1u))
+                    for (int q = 1; q <= 3; ++q) {
+                        o[-(long long)q * sz] = val.x;
+                        if (fl & 2u) o[-(long long)q * sz + 1] = val.y;
+                    }
+                if (k == L.nz - 1 && !(L.io & kHaloZHi) && (fl & 1u))
+                    for (int q = 1; q <= 3; ++q) {
+                        o[(long long)q * sz] = val.x;
+                        if (fl & 2u) o[(long long)q * sz + 1] = val.y;
+                    }
             }
             if (volume) {
                 // smoothed Heaviside in FP64 (src/fluid_update_fsf.cpp:50-71)
                 const double PI_REF = 3.14159265359;
-                const int nw = act1[r] ? 2 : 1;
-                for (int e = 0; e < nw; ++e) {
+                for (int e = 0; e < 2; ++e) {
+                    if (!(fl & (e ? 2u : 1u))) continue;
                     const double ph = e ? val.y : val.x;
                     double H = 0.0;
                     if (ph > a.psi) H = 1.0;
@@ -678,20 +725,23 @@ __device__ __forceinline__ bool tile_item(const CUtensorMap* tmap, const TileArg
             partial_out[1] = sb2;
         }
     }
-    // every wait of the item has completed: retire the barriers
-    __syncthreads();
-    if (tid == 0)
-        for (int s = 0; s < RING; ++s) mbar_inval(bar + s);
-    __syncthreads();
+    if (REUSE) {
+        // every wait of the item has completed: retire the barriers
+        __syncthreads();
+        if (tid == 0)
+            for (int s = 0; s < RING; ++s) mbar_inval(bar + s);
+        __syncthreads();
+    }
     return true;
 }
 
 template <class C, bool REINI, int STAGE, bool VOLUME, bool ISO>
-__global__ void __launch_bounds__(C::NT, C::MINB) tile_kernel(const __grid_constant__ CUtensorMap tmap, TileArgs a) {
+__global__ void __launch_bounds__(C::NT, C::MINB) tile_kernel(const __grid_constant__ CUtensorMap tmap,
+                                                              const __grid_constant__ TileArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ double red_a[C::NW], red_b[C::NW];
     const long long b = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    tile_item<C, REINI, STAGE, ISO>(&tmap, a, blockIdx.x, blockIdx.y, blockIdx.z, VOLUME, smem_raw, red_a, red_b,
+    tile_item<C, REINI, STAGE, ISO, false>(&tmap, a, blockIdx.x, blockIdx.y, blockIdx.z, VOLUME, smem_raw, red_a, red_b,
                                a.partial + 2 * b);
 }
 
@@ -748,7 +798,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) batch_tile_kernel(const TiledM
         // the item's arguments in a thread-local copy: the plane loop reads
         // them across CTA barriers, after which shared memory would be reread
         const TileArgs a = sa;
-        if (!tile_item<C, REINI, STAGE, ISO>(maps + 3 * m + (STAGE - 1), a, bx, by, bz, volume, smem_raw, red_a, red_b,
+        if (!tile_item<C, REINI, STAGE, ISO, true>(maps + 3 * m + (STAGE - 1), a, bx, by, bz, volume, smem_raw, red_a, red_b,
                                         vol_part + 2 * t))
             break;
     }

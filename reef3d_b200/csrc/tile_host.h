@@ -19,7 +19,8 @@ struct TileArgs {
     double* partial;
     int* err;
     float rh[3];
-    float eps[3];    // 1/h^2 per axis
+    float psi1[3];   // 0.3e-6 h^2 and 0.75e-6 h^2 per axis: the WENO psi 1e-6
+    float psi2[3];   // over the indicators' leading coefficients 10/3, 4/3
     double beps[3];  // FP64 interface band: 1e-6 h^2 per axis, h = 1/(double)rh
     float dtr;
     float deltax;
@@ -35,7 +36,8 @@ struct TileArgs {
 // True when the three axes' spacing constants are bitwise equal (cubic
 // cells): the kernels then hold one set for all axes, with the same results.
 inline bool tile_args_iso(const TileArgs& a) {
-    return a.rh[0] == a.rh[1] && a.rh[1] == a.rh[2] && a.eps[0] == a.eps[1] && a.eps[1] == a.eps[2];
+    return a.rh[0] == a.rh[1] && a.rh[1] == a.rh[2] && a.psi1[0] == a.psi1[1] && a.psi1[1] == a.psi1[2] &&
+           a.psi2[0] == a.psi2[1] && a.psi2[1] == a.psi2[2] && a.beps[0] == a.beps[1] && a.beps[1] == a.beps[2];
 }
 
 // A member of a batch that runs on the tiled kernels (3D, uniform, FP32).
