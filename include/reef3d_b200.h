@@ -415,7 +415,7 @@ int r3d_init_spheres_tg(r3d_handle* h, int nspheres, const double* spheres, int 
  *  R3D_OPT_TILED  1 = TMA-tiled FP32x2 stage kernels on 3D uniform FP32
  *                 grids (default), 0 = one-cell-per-thread kernels;
  *                 reading it returns whether the tiled path is in use.
- *  R3D_OPT_CHUNK  z-planes per CTA of the tiled kernels (default 16); sets
+ *  R3D_OPT_CHUNK  z-planes per CTA of the tiled kernels (default: by size); sets
  *                 both stage kinds, R3D_OPT_CHUNK_REINIT then sets the
  *                 reinitialisation stages' alone (reading CHUNK returns the
  *                 convection stages' value).

@@ -436,6 +436,8 @@ int r3d_create(const r3d_grid_desc* desc, r3d_handle** out) {
     h->desc = *desc;
     h->desc.xn = h->desc.yn = h->desc.zn = nullptr;
     cudaGetDevice(&h->device);
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) == cudaSuccess && sms > 0) h->sms = sms;
     h->L = make_layout(desc->nx, desc->ny, desc->nz);
     build_metrics(desc->nx, desc->ny, desc->nz, desc->xn, desc->yn, desc->zn, desc->f45, h->M);
 
@@ -494,6 +496,8 @@ int r3d_create(const r3d_grid_desc* desc, r3d_handle** out) {
     bool h_ok = true;
     for (int a = 0; a < 3; ++a) h_ok = h_ok && h->M.h[a] > 1.0e-14 && h->M.h[a] < 1.0e14;
     if (fp32(h) && !h->L.two_d && h->M.uniform && h_ok && h->L.ncell < (1ll << 31)) {
+        tile_default(h->L, h->sms, false, &h->tile_cfg, &h->kc);
+        tile_default(h->L, h->sms, true, &h->tile_cfg_r, &h->kc_r);
         std::string why;
         const int ids[3] = {R3D_PHI, R3D_WORK1, R3D_WORK2};
         bool ok = true;
@@ -1378,9 +1382,6 @@ int r3d_set_velocity_airy(r3d_handle* h, double amplitude, double wavelength, do
         }
         R3D_CUDA(h, cudaMemcpy(h->coord, c.data(), c.size() * sizeof(double), cudaMemcpyHostToDevice));
     }
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) == cudaSuccess && sms > 0)
-        h->sms = sms;
     const double kw = 2.0 * 3.141592653589793 / wavelength;
     const double om = std::sqrt(gravity * kw * std::tanh(kw * depth));
     h->ap = r3d::AiryParams{amplitude * om / std::sinh(kw * depth), kw, om, depth};

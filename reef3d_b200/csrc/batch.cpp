@@ -341,7 +341,7 @@ void save_cache(const char* path) {
 
 // The z chunks and the (tile configuration, z chunk) candidates of the
 // autotuners.
-constexpr int kChunks[] = {6, 7, 8, 10, 12, 16, 32};
+constexpr int kChunks[] = {2, 4, 6, 7, 8, 10, 12, 16, 32};
 
 std::vector<std::pair<int, int>> tile_candidates() {
     std::vector<std::pair<int, int>> out;

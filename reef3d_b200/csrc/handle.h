@@ -60,7 +60,8 @@ struct r3d_handle {
     bool tile_ok = false;
     int use_tile = 1;
     // tile configuration (shape, rows per thread, ring depth) and z chunk of
-    // the convection stages; *_r: of the reinitialisation stages
+    // the convection stages; *_r: of the reinitialisation stages (from
+    // tile_default when the instance runs on tiles)
     int kc = 16;
     int tile_cfg = 0;
     int kc_r = 16;

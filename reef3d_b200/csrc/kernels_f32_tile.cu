@@ -971,6 +971,37 @@ int tile_cfg_describe(int cfg, int* tx, int* ty, int* ry, int* ring, int* thread
 
 int tile_ctas_per_sm(int cfg) { return info(cfg).minb; }
 
+// Measured over every configuration and chunk on grids from 32^3 to
+// 512 x 128 x 256 (us per stage, this choice / the best of the sweep /
+// configuration 0 with 16 planes, the former default):
+//   convection        64^3 7.4 / 6.7 / 20   128^3 21.3 / 20.6 / 26
+//                     96^3 12.7 / 12.0 / 22  201x97x153 34 / 34 / 40  256^3 122 / 122 / 150
+//   reinitialisation  64^3 10.3 / 8.8 / 45  128^3 27.7 / 27.2 / 50
+//                     201x97x153 43 / 43 / 63  256^3 133 / 133 / 165
+// Shape: the 64 x 8 tile for the convection (four CTAs per SM; it spills in
+// the 96 registers of the fifth), 32 x 16 at five CTAs for the
+// reinitialisation, or the other shape where it pads the grid less.  Chunk:
+// a plane takes about 1 us alone on an SM and 2 us beside three others, an
+// item 4 us on top, so the chunk shrinks until the items fill the device
+// about twice over; the reinitialisation's items hold unequal numbers of FP64
+// band cells and want three times as many.
+void tile_default(const Layout& L, int sms, bool reini, int* cfg, int* kc) {
+    auto columns = [&](int c) {
+        return (long long)((L.nx + info(c).tx - 1) / info(c).tx) * ((L.ny + info(c).ty - 1) / info(c).ty);
+    };
+    auto padded = [&](int c) { return columns(c) * info(c).tx * info(c).ty; };
+    const int first = reini ? 6 : 1, other = reini ? 1 : 3;
+    *cfg = 100 * padded(other) < 97 * padded(first) ? other : first;
+    tile_default_chunk(columns(*cfg) * L.nz, sms, *cfg, reini, kc);
+}
+
+void tile_default_chunk(long long planes, int sms, int cfg, bool reini, int* kc) {
+    const double waves = (double)planes / ((double)sms * info(cfg).minb);  // of one-plane items
+    const int want = (int)(waves / (reini ? 7.0 : 2.2) + 0.5);
+    const int lo = reini ? 1 : 2, hi = reini ? 8 : 10;
+    *kc = want < lo ? lo : want > hi ? hi : want;
+}
+
 // Sets the attributes of every instantiation once per device.
 bool tile_prepare() {
     static bool done[64] = {};
