@@ -182,7 +182,10 @@ __global__ void __launch_bounds__(256) vmax_f32_kernel(Layout L, const float* __
 // dt = N47 * MIN(1e10, 2/(sqrt(umax^2+vmax^2+wmax^2)/dx + sqrt(0/dx)))
 // (src/ietimestep.cpp:160-188 with maxF=maxG=maxH=0, evaluated at the
 // smallest cell length, where the reference's minimum over cells sits).
-__global__ void dt_kernel(const unsigned long long* vm, const double* vscale, double dxmin, double n47, double* dt) {
+// reset: the maxima of u and w start from 0 again (the Airy generator's next
+// step finds new ones; v keeps its own).
+__global__ void dt_kernel(unsigned long long* vm, const double* vscale, double dxmin, double n47, double* dt,
+                          bool reset) {
     // max |s*u| = |s| * max |u| exactly: rounding is monotone
     const double sc = fabs(*vscale);
     const double umax = sc * __longlong_as_double((long long)vm[0]);
@@ -192,6 +195,7 @@ __global__ void dt_kernel(const unsigned long long* vm, const double* vscale, do
     const double cand = 2.0 / ((sqrt(umax * umax + vmax * vmax + wmax * wmax)) / dxmin + sqrt((4.0 * fabs(0.0)) / dxmin));
     cu = cu < cand ? cu : cand;
     *dt = n47 * cu;
+    if (reset) vm[0] = vm[2] = 0;
 }
 
 // --------------------------------------------------------------- volume
@@ -272,10 +276,17 @@ __global__ void volume_direct_kernel(Layout L, const T* __restrict__ phi, const 
 // separable, so each block first tabulates the x and z factors in shared
 // memory (coord: x centres, x faces, z centres, z faces of padded indices
 // -3..n+2) and then writes rows with two multiplies per value.
-template <typename T>
+// Bound by the stores: a thread writes 16 bytes of u and of w, aligned (the
+// row from its padding slot on), where one value a thread at an odd offset
+// reached 2.3 TB/s.  MAX: also the CFL maxima of the faces written (those of
+// vmax_kernel; the largest product of a row is formed anyway), into vmax[0]
+// and vmax[2], which saves the CFL step's reading of three fields: at 1024 x
+// 128 x 256 FP32 the two took 119 + 75 us.
+template <typename T, bool MAX>
 __global__ void __launch_bounds__(256) airy_kernel(Layout L, T* __restrict__ u, T* __restrict__ w,
                                                    const double* __restrict__ coord, const double* __restrict__ t,
-                                                   AiryParams ap) {
+                                                   AiryParams ap, unsigned long long* vmax) {
+    constexpr int V = 16 / (int)sizeof(T);
     extern __shared__ double tab[];
     const int nx6 = L.nx + 6, nz6 = L.nz + 6;
     double* xu = tab;
@@ -293,14 +304,50 @@ __global__ void __launch_bounds__(256) airy_kernel(Layout L, T* __restrict__ u, 
         zw[k] = ap.a * sinh(ap.kw * fmin(coord[2 * nx6 + nz6 + k], ap.depth));
     }
     __syncthreads();
-    const int py = L.two_d ? 1 : L.ny + 6;
-    const long long rows = (long long)py * nz6;
-    for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
+    const int py = L.two_d ? 1 : L.ny + 6, nq = L.px / V;
+    const long long items = (long long)py * nz6 * nq;
+    double mu = 0.0, mw = 0.0;
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < items;
+         e += (long long)gridDim.x * blockDim.x) {
+        const int q = (int)(e % nq);
+        const long long r = e / nq;
         const int jj = (int)(r % py), kk = (int)(r / py);
-        const long long base = (long long)kk * L.sz + (long long)jj * L.sy + (L.gx - 3);
-        for (int i = threadIdx.x; i < nx6; i += blockDim.x) {
-            u[base + i] = static_cast<T>(zu[kk] * xu[i]);
-            w[base + i] = static_cast<T>(zw[kk] * xw[i]);
+        const long long base = (long long)kk * L.sz + (long long)jj * L.sy + V * q;
+        alignas(16) T fu[V];
+        alignas(16) T fw[V];
+        const bool row = L.two_d || (jj >= 3 && jj < L.ny + 3);
+        const bool inu = row && kk >= 3 && kk < L.nz + 3;
+        const bool inw = row && kk >= 3 && kk < L.nz + 3 - ((L.io & kHaloZHi) ? 0 : 1);
+#pragma unroll
+        for (int m = 0; m < V; ++m) {
+            const int s = V * q + m, i = s - 1;  // row slot 1 is padded index -3; padding gets 0
+            const bool in = i >= 0 && i < nx6;
+            fu[m] = in ? static_cast<T>(zu[kk] * xu[i]) : T(0);
+            fw[m] = in ? static_cast<T>(zw[kk] * xw[i]) : T(0);
+            if (MAX && s >= L.gx && s < L.gx + L.nx) {
+                if (inu && s < L.gx + L.nx - 1) mu = fmax(mu, fabs((double)fu[m]));
+                if (inw) mw = fmax(mw, fabs((double)fw[m]));
+            }
+        }
+        *reinterpret_cast<float4*>(u + base) = *reinterpret_cast<const float4*>(fu);
+        *reinterpret_cast<float4*>(w + base) = *reinterpret_cast<const float4*>(fw);
+    }
+    if (MAX) {
+        for (int o = 16; o > 0; o >>= 1) {
+            mu = fmax(mu, __shfl_down_sync(0xffffffffu, mu, o));
+            mw = fmax(mw, __shfl_down_sync(0xffffffffu, mw, o));
+        }
+        __shared__ double s[2][8];
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        if (lane == 0) { s[0][warp] = mu; s[1][warp] = mw; }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int q = 1; q < (int)(blockDim.x >> 5); ++q) {
+                mu = fmax(mu, s[0][q]);
+                mw = fmax(mw, s[1][q]);
+            }
+            atomicMax(vmax + 0, (unsigned long long)__double_as_longlong(mu));
+            atomicMax(vmax + 2, (unsigned long long)__double_as_longlong(mw));
         }
     }
 }
@@ -797,7 +844,7 @@ int launch_io_ghosts(const Layout& L, void* phi, void* a1, void* a2, bool fp32, 
 }
 
 int launch_dt_from_max(double dxmin, double n47, const Scratch& s, cudaStream_t st) {
-    dt_kernel<<<1, 1, 0, st>>>(s.vmax, s.vscale, dxmin, n47, s.dt);
+    dt_kernel<<<1, 1, 0, st>>>(s.vmax, s.vscale, dxmin, n47, s.dt, false);
     return 1;
 }
 
@@ -922,15 +969,22 @@ int launch_netvol(const Scratch& s, double qi, double qo, cudaStream_t st) {
 size_t airy_smem_bytes(const Layout& L) { return (size_t)(2 * (L.nx + 6) + 2 * (L.nz + 6)) * sizeof(double); }
 
 int launch_airy(const Layout& L, void* u, void* w, bool fp32, const double* coord, const double* t,
-                const AiryParams& ap, int sms, cudaStream_t st) {
-    const long long rows = (long long)(L.two_d ? 1 : L.ny + 6) * (L.nz + 6);
-    const int grid = (int)(rows < 4LL * sms ? rows : 4LL * sms);
+                const AiryParams& ap, int sms, unsigned long long* vmax, cudaStream_t st) {
+    const long long items =
+        (long long)(L.two_d ? 1 : L.ny + 6) * (L.nz + 6) * (L.px / (fp32 ? 4 : 2));
+    const long long blocks = (items + 255) / 256;
+    const unsigned grid = (unsigned)(blocks < 8LL * sms ? blocks : 8LL * sms);
     const size_t smem = airy_smem_bytes(L);
-    if (fp32)
-        airy_kernel<float><<<grid, 256, smem, st>>>(L, static_cast<float*>(u), static_cast<float*>(w), coord, t, ap);
-    else
-        airy_kernel<double><<<grid, 256, smem, st>>>(L, static_cast<double*>(u), static_cast<double*>(w), coord, t,
-                                                     ap);
+#define R3D_AIRY(T, M) \
+    airy_kernel<T, M><<<grid, 256, smem, st>>>(L, static_cast<T*>(u), static_cast<T*>(w), coord, t, ap, vmax)
+    if (fp32) {
+        if (vmax) R3D_AIRY(float, true);
+        else R3D_AIRY(float, false);
+    } else {
+        if (vmax) R3D_AIRY(double, true);
+        else R3D_AIRY(double, false);
+    }
+#undef R3D_AIRY
     return 1;
 }
 
@@ -938,10 +992,11 @@ int airy_prepare(const Layout& L) {
     const size_t smem = airy_smem_bytes(L);
     if (smem > 227 * 1024) return 1;
     if (smem > 48 * 1024) {
-        if (cudaFuncSetAttribute(airy_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(airy_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-                cudaSuccess)
+        auto allow = [&](auto* k) {
+            return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+        };
+        if (!allow(airy_kernel<float, false>) || !allow(airy_kernel<float, true>) ||
+            !allow(airy_kernel<double, false>) || !allow(airy_kernel<double, true>))
             return 1;
     }
     return 0;
@@ -1010,8 +1065,8 @@ int launch_ghost_fill(const Layout& L, void* f, bool fp32, cudaStream_t st) {
     return 1;
 }
 
-int launch_cfl(const Layout& L, const void* u, const void* v, const void* w, bool fp32, double dxmin, double n47,
-               const Scratch& s, cudaStream_t st) {
+int launch_vmax(const Layout& L, const void* u, const void* v, const void* w, bool fp32, const Scratch& s,
+                cudaStream_t st) {
     cudaMemsetAsync(s.vmax, 0, 3 * sizeof(unsigned long long), st);
     const long long rows = (long long)L.ny * L.nz;
     const dim3 grid((unsigned)(rows < 1184 ? rows : 1184)), block(256);
@@ -1023,8 +1078,17 @@ int launch_cfl(const Layout& L, const void* u, const void* v, const void* w, boo
     } else
         vmax_kernel<double><<<grid, block, 0, st>>>(L, static_cast<const double*>(u), static_cast<const double*>(v),
                                                     static_cast<const double*>(w), s.vmax);
-    dt_kernel<<<1, 1, 0, st>>>(s.vmax, s.vscale, dxmin, n47, s.dt);
-    return 2;
+    return 1;
+}
+
+int launch_dt(double dxmin, double n47, const Scratch& s, bool reset, cudaStream_t st) {
+    dt_kernel<<<1, 1, 0, st>>>(s.vmax, s.vscale, dxmin, n47, s.dt, reset);
+    return 1;
+}
+
+int launch_cfl(const Layout& L, const void* u, const void* v, const void* w, bool fp32, double dxmin, double n47,
+               const Scratch& s, cudaStream_t st) {
+    return launch_vmax(L, u, v, w, fp32, s, st) + launch_dt(dxmin, n47, s, false, st);
 }
 
 int launch_volume_reduce(const Layout&, const Scratch& s, long long nblocks, double period, cudaStream_t st) {

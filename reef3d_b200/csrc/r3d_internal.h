@@ -175,8 +175,9 @@ struct AiryParams {
 // -3..n+2).  airy_prepare sets the kernels' shared-memory limit (nonzero:
 // the grid is too long in x or z for the shared-memory tables).
 int airy_prepare(const Layout& L);
+// vmax: where the CFL maxima of u and w go (s.vmax), or null.
 int launch_airy(const Layout& L, void* u, void* w, bool fp32, const double* coord, const double* t,
-                const AiryParams& ap, int sms, cudaStream_t st);
+                const AiryParams& ap, int sms, unsigned long long* vmax, cudaStream_t st);
 
 // Fluid constants of fluid_update_fsf (W1..W4, src/ini.cpp:831-834).
 struct FluidConst {
@@ -205,6 +206,11 @@ int launch_volume_direct_clock(const Layout& L, const void* phi, bool fp32, cons
                                const Scratch& s, cudaStream_t st);
 int launch_cfl(const Layout& L, const void* u, const void* v, const void* w, bool fp32,
                double dxmin, double n47, const Scratch& s, cudaStream_t st);
+// Its two halves: the face maxima into s.vmax; dt from them (reset: u's and
+// w's maxima start from 0 again).
+int launch_vmax(const Layout& L, const void* u, const void* v, const void* w, bool fp32, const Scratch& s,
+                cudaStream_t st);
+int launch_dt(double dxmin, double n47, const Scratch& s, bool reset, cudaStream_t st);
 int launch_ghost_fill(const Layout& L, void* f, bool fp32, cudaStream_t st);
 
 // ioflow_f level-set hooks (src/ioflow_waterlevel.cpp:29-177) on an
