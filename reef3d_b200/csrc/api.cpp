@@ -173,7 +173,6 @@ int ensure_staging(r3d_handle* h) {
     const size_t need = sizeof(double) * (size_t)(h->L.nx + 6) * (h->L.ny + 6) * (h->L.nz + 6);
     if (h->staging_bytes >= need) return R3D_OK;
     if (h->staging) cudaFree(h->staging);
-    if (h->coord) cudaFree(h->coord);
     h->staging = nullptr;
     h->staging_bytes = 0;
     if (cudaMalloc(&h->staging, need) != cudaSuccess) {
