@@ -1,0 +1,179 @@
+"""Stage kernels, run loop and host copies at the sizes and values where they
+switch paths: the dealing of interface-band cells, steep fields, the FP64
+weights outside their fast range, the default tiles, the CFL maxima shared by
+a run's steps, and pageable copies around the piece size."""
+import numpy as np
+import pytest
+
+import reef3d_b200 as r3d
+from test_gpu_parity import relmax
+from test_oracle_golden import interior, visible_mask
+
+pytestmark = pytest.mark.gpu
+
+FLAGS = dict(f43=0.5, f44=2, f45=2.1, f49=1, n47=0.125)
+EPS32 = 2.0 ** -24
+
+
+def instance(dims, precision=r3d.FP32, nodes=None, **kw):
+    return r3d.LevelSet(*dims, *(nodes or ()), precision=precision, **dict(FLAGS, **kw))
+
+
+def dense(ls):
+    return ls.download(r3d.PHI, r3d.LAYOUT_DENSE)
+
+
+@pytest.mark.parametrize("f49", [1, 0])
+@pytest.mark.parametrize("cells", [1, 3, 10, 11, 20, 21, 32, 64])
+def test_band_cells_dealt_to_lanes(cells, f49):
+    """A sheet that crosses `cells` cells of every row of 64 (one axis per lane
+    up to twenty cells of a warp's rows, three beyond): the tiled kernels
+    against the one-cell-per-thread ones.  Both form the band in FP64, so a
+    cell differs by the rounding of the other cells' FP32 right-hand sides:
+    two pseudo-steps of dtau <= h, RHS errors of a few ulp of 1."""
+    n = 64
+    x = (np.arange(n) + 0.5) / n
+    rng = np.random.default_rng(cells)
+    phi = np.broadcast_to(x[:, None, None] - 0.5, (n, n, n)).copy()
+    # the sheet lies on a plane z = const over `cells` columns, elsewhere above
+    phi[:, :, cells:] += 4.0 / n
+    phi += 1e-3 / n * rng.standard_normal(phi.shape)
+    out = []
+    for tiled in (1, 0):
+        with instance((n, n, n), f49=f49) as ls:
+            ls.set_option(r3d.OPT_TILED, tiled)
+            ls.upload(r3d.PHI, phi, r3d.LAYOUT_DENSE)
+            ls.ghost_fill()
+            ls.reinit(1)
+            ls.sync()
+            out.append(dense(ls))
+    h = 1.0 / n
+    assert np.max(np.abs(out[0] - out[1])) <= 3 * h * 64 * EPS32 + 2 * EPS32
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e2, 1e4, 1e7])
+@pytest.mark.parametrize("tiled", [1, 0])
+def test_steep_fields_fp32(scale, tiled):
+    """Gradients up to 1e7: the FP32 weights against FP64's.  The operator is
+    compared relative to its largest value; the smoothness indicators' FP32
+    differences of phi carry |phi| 2^-24 / h against gradients of order 1."""
+    n = 32
+    rng = np.random.default_rng(3)
+    res = []
+    x = (np.arange(n) + 0.5) / n
+    phi = np.sin(5 * x)[None, None, :] * np.cos(4 * x)[None, :, None] + 0.5 * np.sin(6 * x)[:, None, None]
+    phi = scale * (phi + 0.3 * np.sign(phi) + 0.01 * rng.standard_normal(phi.shape))
+    phi = phi.astype(np.float32).astype(np.float64)
+    for prec in (r3d.FP64, r3d.FP32):
+        with instance((n, n, n), prec) as ls:
+            if prec == r3d.FP32:
+                ls.set_option(r3d.OPT_TILED, tiled)
+            ls.init_spheres_tg([(0.5, 0.5, 0.5, 0.2)], [(1, 0.5), (2, 0.25)])
+            ls.upload(r3d.PHI, phi, r3d.LAYOUT_DENSE)
+            ls.ghost_fill()
+            ls.set_dt(1e-3)
+            ls.stage(r3d.STAGE_CONVECTION, 1)
+            ls.sync()
+            res.append(ls.download(r3d.WORK1, r3d.LAYOUT_DENSE))
+    assert np.all(np.isfinite(res[1]))
+    # dt |u| / h of the differences' error: 1e-3 * 1 * 32 * 8 ulp, and phi's own rounding
+    assert relmax(res[1], res[0]) <= 1e-3 * n * 64 * EPS32 + 4 * EPS32
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e20, 1e34, 1e35, 1e36, 1e70, 1e80])
+def test_fp64_weights_range(port_lib, scale):
+    """The FP64 operators bit for bit where the squared indicators pass 2^499
+    (weights_any) and where they do not, mixed in one field."""
+    nx, ny, nz = 20, 11, 14
+    rng = np.random.default_rng(5)
+    xn, yn, zn = (r3d.uniform_nodes(n) for n in (nx, ny, nz))
+    phi = rng.standard_normal((nx + 6, ny + 6, nz + 6))
+    phi[: nx // 2] *= scale
+    u, v, w = (rng.standard_normal(phi.shape) for _ in range(3))
+    o = port_lib(nx, ny, nz, xn, yn, zn, **FLAGS)
+    with instance((nx, ny, nz), r3d.FP64, (xn, yn, zn)) as ls:
+        for f, a in ((r3d.PHI, phi), (r3d.U, u), (r3d.V, v), (r3d.W, w)):
+            ls.upload(f, a)
+        ls.convection_L()
+        got = ls.download(r3d.L)
+        ls.reinidisc_L()
+        got_r = ls.download(r3d.L)
+    for mine, ref in ((got, o.weno_L(phi, u, v, w)), (got_r, o.reinidisc_L(phi))):
+        assert np.array_equal(interior(mine, nx, ny, nz), interior(ref, nx, ny, nz), equal_nan=True)
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2), (33, 17, 5), (64, 8, 1), (65, 9, 40), (96, 96, 96)])
+def test_default_tiles(dims):
+    """The size-dependent default gives the level set of any other choice."""
+    out = []
+    for pick in (None, (1, 10), (0, 16)):
+        with instance(dims) as ls:
+            ls.init_spheres_tg([(0.5, 0.4, 0.6, 0.2), (0.3, 0.6, 0.3, 0.1)], [(1, 0.5), (2, -0.3)])
+            assert ls.get_option(r3d.OPT_TILED) == 1 and ls.get_option(r3d.OPT_CHUNK) >= 1
+            if pick:
+                ls.set_option(r3d.OPT_TILE_CFG, pick[0])
+                ls.set_option(r3d.OPT_CHUNK, pick[1])
+            ls.run(2)
+            ls.sync()
+            out.append(dense(ls))
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("precision", [r3d.FP32, r3d.FP64])
+@pytest.mark.parametrize("dims", [(40, 24, 18), (48, 1, 37)])
+@pytest.mark.parametrize("airy", [False, True])
+def test_run_shares_cfl_maxima(precision, dims, airy):
+    """An adaptive run's time steps are those of single steps with r3d_cfl_dt
+    before each, for stored velocities (scaled by the clock), the Airy
+    generator (beside an uploaded v), and velocities uploaded between runs."""
+    def make():
+        ls = instance(dims, precision)
+        ls.init_spheres_tg([(0.5, 0.5, 0.5, 0.25)], [(1, 0.5), (2, 0.3)])
+        if airy:
+            ls.set_time(0.0)
+            ls.set_velocity_airy(0.05, 2.0, 0.5)
+            ls.upload(r3d.V, np.full(ls.reef3d_shape, 0.01))
+        else:
+            ls.set_velocity_period(1.0)
+            ls.set_time(0.1)
+        return ls
+    shape = (dims[0] + 6, dims[1] + 6, dims[2] + 6)
+    faster = np.random.default_rng(1).standard_normal(shape)
+    a, b = make(), make()
+    try:
+        for field in (None, r3d.W, r3d.U):
+            for ls in (a, b):
+                if field is not None and not airy:
+                    ls.upload(field, 3.0 * faster)
+            a.run(3)
+            for _ in range(3):
+                b.step(b.cfl_dt())
+            assert a.time() == b.time()
+            assert np.array_equal(dense(a), dense(b))
+    finally:
+        a.close()
+        b.close()
+
+
+@pytest.mark.parametrize("nz", [11, 12, 24, 61, 128])
+@pytest.mark.parametrize("precision", [r3d.FP64, r3d.FP32])
+def test_pageable_copies(nz, precision):
+    """Host arrays below, at and beyond the size from which pageable copies
+    are split (4 MiB, in 1 MiB pieces), against a pinned array in one copy;
+    nx ny chosen so that 11 and 12 planes lie either side of 4 MiB."""
+    import torch
+    nx, ny = 220, 208
+    a = np.random.default_rng(nz).standard_normal((nz, ny, nx)).astype(np.float32).astype(np.float64)
+    pin = torch.empty(a.shape, dtype=torch.float64, pin_memory=True)
+    with instance((nx, ny, nz), precision) as ls:
+        ls.upload(r3d.PHI, a, r3d.LAYOUT_DENSE)
+        ls.download_ptr(r3d.PHI, pin.data_ptr(), r3d.LAYOUT_DENSE)
+        assert np.array_equal(pin.numpy(), a)
+        pin *= 2.0
+        ls.upload_ptr(r3d.PHI, pin.data_ptr(), r3d.LAYOUT_DENSE)
+        assert np.array_equal(dense(ls), 2.0 * a)
+        r = np.random.default_rng(1).standard_normal(ls.reef3d_shape).astype(np.float32).astype(np.float64)
+        ls.upload(r3d.U, r)
+        m = visible_mask(nx, ny, nz)
+        got = ls.download(r3d.U)
+        assert np.array_equal(got[m], r[m]) and not np.any(got[~m])
