@@ -10,10 +10,12 @@ namespace r3d {
 namespace {
 
 constexpr int kBX = 32, kBY = 4;
-// resident blocks per SM the stage kernels are register-limited for
-#ifndef R3D_F64_MINB
-#define R3D_F64_MINB 8
-#endif
+// Resident blocks per SM the stage kernels are register-limited for: 64
+// registers in the convection; 80 in the reinitialisation, which holds the six
+// face differences of an axis through the weights and spills in 64 (256^3,
+// us per stage 1 / 2: 776 / 744 at eight blocks against 816 / 847 at six;
+// 813 / 854 at six against 926 / 954 at eight).
+constexpr int kConvBlocks = 8, kReiniBlocks = 6;
 
 struct StageArgs {
     const double* fn;   // step start value (phi^n / f): read at the cell only
@@ -102,7 +104,7 @@ __device__ __forceinline__ void heaviside_volume(const KGrid<double>& g, double 
 // Reinit stage s of src/reini_RK3.cpp:113-137: the same with the per-cell
 // pseudo time step.
 template <bool TWO_D, int STAGE, bool REINI, bool VOLUME, bool DF = false>
-__global__ void __launch_bounds__(kBX * kBY, R3D_F64_MINB) stage_kernel(KGrid<double> g, StageArgs a) {
+__global__ void __launch_bounds__(kBX * kBY, REINI ? kReiniBlocks : kConvBlocks) stage_kernel(KGrid<double> g, StageArgs a) {
     int i, j, k;
     cell_of_thread(g.L, TWO_D, i, j, k);
     const bool active = i < g.L.nx && j < g.L.ny && k < g.L.nz;

@@ -28,21 +28,58 @@ __device__ __forceinline__ double div_rn(double a, double b, double r) {
     return fma(fma(-b, q1, a), r, q1);
 }
 
+// 1/b to within an ulp for a normal b: the hardware's approximation (relative
+// error e below 2^-23) and one cubic Newton step y (1 + e + e^2), whose error
+// is e^3.
+__device__ __forceinline__ double rcp_f64(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
+// a / b from y, an approximation of 1/b to a few ulps: the quotient a y
+// corrected once by its residual, which a fused multiply-add gives exactly
+// (Markstein, as in div_rn).  Before its last rounding the result is within
+// 2^-102 of a/b relative to it, so it is the IEEE quotient unless a/b lies
+// that close to the middle of two doubles (one in 2^49 random quotients).
+__device__ __forceinline__ double div_y(double a, double b, double y) {
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+
+__device__ __forceinline__ double2 ldg2(const double* p) { return __ldg(reinterpret_cast<const double2*>(p)); }
+
+// The nonlinear weights c_r / (s_r^2 sum), sum = c0/s0^2 + c1/s1^2 + c2/s2^2,
+// by the compiler's divisions: any A = s0^2, B = s1^2, C = s2^2 (overflowed,
+// infinite, NaN).
+__device__ __noinline__ void weights_any(double c0, double c1, double c2, double A, double B, double C, double* w) {
+    const double eps = 0.0;
+    const double sum = c0 / A + c1 / B + c2 / C;
+    w[0] = c0 / (eps + A * sum);
+    w[1] = c1 / (eps + B * sum);
+    w[2] = c2 / (eps + C * sum);
+}
+
 // WENO5 derivative from the divided differences q1..q5 of the upwind set,
 // node tables of index t and the side: the record W = wt + 18 (2t + side)
 // holds Q0..Q5, C0..C2, S0..S8 (16-byte aligned: nine 16-byte loads).
 // Minus side: IS src/weno_nug_func.h:48-60, weights :133-143,
 // reconstruction src/weno_hj_df_nug.cpp:155-159.  Plus side: :61-73,
 // :144-153, :186-190.  epsilon = 0, psi = 1e-6 (src/weno_nug_func.cpp:26).
-__device__ __forceinline__ double2 ldg2(const double* p) { return __ldg(reinterpret_cast<const double2*>(p)); }
-
+//
+// The six quotients of the weights have 1/A, 1/B, 1/C and 1/sum in common
+// (1/(A sum) = 1/A 1/sum to a few ulps): four reciprocals and 33 FP64
+// operations without range checks, where six IEEE divisions took about 50
+// and 60 others.  Where one of A, B, C (1e-12 and up by psi) leaves
+// [2^-511, 2^499), compared on the high words, weights_any forms them.
 __device__ __forceinline__ double weno5(const double* __restrict__ W, bool plus, double q1, double q2, double q3,
                                         double q4, double q5) {
     const double2 w01 = ldg2(W + 0), w23 = ldg2(W + 2), w45 = ldg2(W + 4), w67 = ldg2(W + 6);
     const double2 w89 = ldg2(W + 8), wab = ldg2(W + 10), wcd = ldg2(W + 12), wef = ldg2(W + 14);
     const double2 wgh = ldg2(W + 16);
     const double S[9] = {w89.y, wab.x, wab.y, wcd.x, wcd.y, wef.x, wef.y, wgh.x, wgh.y};
-    const double psi = 1.0e-6, eps = 0.0;
+    const double psi = 1.0e-6;
     const double dq12 = q1 - q2, dq23 = q2 - q3, dq32 = q3 - q2;
     const double dq34 = q3 - q4, dq43 = q4 - q3, dq54 = q5 - q4;
     const double is1 = S[0] * dq54 * dq54 + S[1] * (dq54) * (dq34) + S[2] * dq34 * dq34;
@@ -50,10 +87,25 @@ __device__ __forceinline__ double weno5(const double* __restrict__ W, bool plus,
     const double is3 = S[6] * dq12 * dq12 + S[7] * (dq32) * (dq12) + S[8] * dq32 * dq32;
     const double a = is1 + psi, b = is2 + psi, c = is3 + psi;
     const double c0 = w67.x, c1 = w67.y, c2 = w89.x;
-    const double sum = c0 / (a * a) + c1 / (b * b) + c2 / (c * c);
-    const double w1 = c0 / (eps + (a * a) * sum);
-    const double w2 = c1 / (eps + (b * b) * sum);
-    const double w3 = c2 / (eps + (c * c) * sum);
+    const double A = a * a, B = b * b, C = c * c;
+    double w1, w2, w3;
+    const unsigned lo = 0x20000000u;  // high word of 2^-511
+    const unsigned top = max(max((unsigned)__double2hiint(A) - lo, (unsigned)__double2hiint(B) - lo),
+                             (unsigned)__double2hiint(C) - lo);
+    if (top < 0x5f200000u - lo) {  // all from 2^-511 to below 2^499
+        const double yA = rcp_f64(A), yB = rcp_f64(B), yC = rcp_f64(C);
+        const double sum = div_y(c0, A, yA) + div_y(c1, B, yB) + div_y(c2, C, yC);
+        const double ys = rcp_f64(sum);
+        w1 = div_y(c0, A * sum, yA * ys);
+        w2 = div_y(c1, B * sum, yB * ys);
+        w3 = div_y(c2, C * sum, yC * ys);
+    } else {
+        double w[3];
+        weights_any(c0, c1, c2, A, B, C, w);
+        w1 = w[0];
+        w2 = w[1];
+        w3 = w[2];
+    }
     const double Q0 = w01.x, Q1 = w01.y, Q2 = w23.x, Q3 = w23.y, Q4 = w45.x, Q5 = w45.y;
     // The two sides' reconstructions differ only in which differences enter
     // and in two signs (minus side :155-159, plus side :186-190); selecting
