@@ -41,9 +41,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_inval(uint64_t* bar) {
-    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
@@ -254,11 +251,9 @@ R3D_TILE_CFGS(R3D_CFG_TYPE)
 #undef R3D_CFG_TYPE
 
 // One work item: the TX x TY column (bx, by) over planes [bz*kc, bz*kc+kc)
-// of one instance.  Returns false when a bounded wait gave up (the error
-// flag is raised and the copies in flight have been waited for).  The
-// item's volume partials (when `volume`) go to partial_out[0..1].  The
-// mbarriers are initialised at the start of the item and invalidated at its
-// end, so a persistent CTA can run items back to back.
+// of one instance.  When a bounded wait gives up, the error flag is raised
+// and the copies in flight are waited for.  The item's volume partials (when
+// `volume`) go to partial_out[0..1].
 // ISO: the three axes have bitwise-equal spacing constants (cubic cells), so
 // axis 0's are used for all three and held once.
 //
@@ -270,8 +265,8 @@ R3D_TILE_CFGS(R3D_CFG_TYPE)
 // release counter), so that warps drift apart where their work differs
 // (interface-band cells in FP64, wall ghosts) instead of meeting at a CTA
 // barrier every plane.
-template <class C, bool REINI, int STAGE, bool ISO, bool REUSE>
-__device__ __forceinline__ bool tile_item(const CUtensorMap* tmap, const TileArgs& a, int bx, int by, int bz,
+template <class C, bool REINI, int STAGE, bool ISO>
+__device__ __forceinline__ void tile_item(const CUtensorMap* tmap, const TileArgs& a, int bx, int by, int bz,
                                           bool volume, unsigned char* smem_raw, double* red_a, double* red_b,
                                           double* partial_out) {
     constexpr int RY = C::RY, BX = C::BX, RING = C::RING, SLOT = C::SLOT;
@@ -709,7 +704,7 @@ __device__ __forceinline__ bool tile_item(const CUtensorMap* tmap, const TileArg
                 mbar_wait_bounded(bar + (q % RING), (uint32_t)((q / RING) & 1));
             }
         }
-        return false;
+        return;
     }
     if (volume) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -725,14 +720,6 @@ __device__ __forceinline__ bool tile_item(const CUtensorMap* tmap, const TileArg
             partial_out[1] = sb2;
         }
     }
-    if (REUSE) {
-        // every wait of the item has completed: retire the barriers
-        __syncthreads();
-        if (tid == 0)
-            for (int s = 0; s < RING; ++s) mbar_inval(bar + s);
-        __syncthreads();
-    }
-    return true;
 }
 
 template <class C, bool REINI, int STAGE, bool VOLUME, bool ISO>
@@ -741,75 +728,61 @@ __global__ void __launch_bounds__(C::NT, C::MINB) tile_kernel(const __grid_const
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ double red_a[C::NW], red_b[C::NW];
     const long long b = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    tile_item<C, REINI, STAGE, ISO, false>(&tmap, a, blockIdx.x, blockIdx.y, blockIdx.z, VOLUME, smem_raw, red_a, red_b,
+    tile_item<C, REINI, STAGE, ISO>(&tmap, a, blockIdx.x, blockIdx.y, blockIdx.z, VOLUME, smem_raw, red_a, red_b,
                                a.partial + 2 * b);
 }
 
-// Persistent batched form: CTAs take the work items of all tiled members
-// (member m owns items [tile0[m], tile0[m+1]); item = (bx, by, bz) of that
-// member) one at a time from a global counter, so CTAs whose items hold
-// more work (FP64 interface band, wall ghosts) take fewer of them.  The
-// last CTA to leave resets the counter pair work[0..1] for the next launch
-// on the stream.  Reinitialisation pseudo-step q is skipped by members with
+// Batched form: CTA t takes item t of the tiled members (member m owns items
+// [tile0[m], tile0[m+1]); item = (bx, by, bz) of that member), so the
+// hardware hands a CTA that is done its SM's next item, whatever the items'
+// work (FP64 interface band, wall ghosts); items taken by persistent CTAs
+// from a counter paid a counter round trip, the retirement of the barriers
+// and three CTA barriers each: 16 members of 64..160 cells an edge 1.64 ->
+// 1.50 ms per step.  Reinitialisation pseudo-step q is skipped by members with
 // f44 <= q; the last stage of a member's step adds its volume partials.
 template <class C, bool REINI, int STAGE, bool ISO>
 __global__ void __launch_bounds__(C::NT, C::MINB) batch_tile_kernel(const TiledMember* __restrict__ members,
                                                                     const CUtensorMap* __restrict__ maps,
                                                                     const long long* __restrict__ tile0, int nm,
-                                                                    int q, double* __restrict__ vol_part,
-                                                                    unsigned* __restrict__ work) {
+                                                                    int q, double* __restrict__ vol_part) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ double red_a[C::NW], red_b[C::NW];
     __shared__ TileArgs sa;
     __shared__ int s_member;
-    __shared__ long long s_t;
-    const long long nt = tile0[nm];
-    for (;;) {
-        if (threadIdx.x == 0) {
-            const long long t0 = (long long)atomicAdd(work, 1u);
-            s_t = t0;
-            if (t0 < nt) {
-                int lo = 0, hi = nm - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (tile0[mid] <= t0) lo = mid;
-                    else hi = mid - 1;
-                }
-                s_member = lo;
-                sa = members[lo].args;
-                sa.out = STAGE == 1 ? members[lo].a1 : STAGE == 2 ? members[lo].a2 : members[lo].phi;
-            }
+    const long long t = blockIdx.x;
+    if (threadIdx.x < 32) {
+        // the last member whose first item is not after t
+        const int lane = threadIdx.x;
+        int m = -1;
+        for (int base = 0; base < nm; base += 32) {
+            const int n = __popc(__ballot_sync(0xffffffffu, base + lane < nm && __ldg(tile0 + base + lane) <= t));
+            m = n ? base + n - 1 : m;
+            if (n < 32) break;
         }
-        __syncthreads();
-        const long long t = s_t;
-        if (t >= nt) break;
-        const int m = s_member;
-        const int f44 = members[m].f44;
-        if (REINI && f44 <= q) {
-            __syncthreads();
-            continue;
-        }
-        const bool volume = STAGE == 3 && (REINI ? q == f44 - 1 : f44 == 0);
-        const long long lt = t - tile0[m];
-        const int ntx = (sa.L.nx + C::TX - 1) / C::TX, nty = (sa.L.ny + C::TY - 1) / C::TY;
-        const int bx = (int)(lt % ntx);
-        const int by = (int)((lt / ntx) % nty);
-        const int bz = (int)(lt / ((long long)ntx * nty));
-        // the item's arguments in a thread-local copy: the plane loop reads
-        // them across CTA barriers, after which shared memory would be reread
-        const TileArgs a = sa;
-        if (!tile_item<C, REINI, STAGE, ISO, true>(maps + 3 * m + (STAGE - 1), a, bx, by, bz, volume, smem_raw, red_a, red_b,
-                                        vol_part + 2 * t))
-            break;
-    }
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(work + 1, 1u) == gridDim.x - 1) {
-            work[0] = 0u;
-            work[1] = 0u;
-            __threadfence();
+        static_assert(sizeof(TileArgs) % sizeof(int) == 0, "copied word by word");
+        const int* src = reinterpret_cast<const int*>(&members[m].args);
+        for (int e = lane; e < (int)(sizeof(TileArgs) / sizeof(int)); e += 32) reinterpret_cast<int*>(&sa)[e] = __ldg(src + e);
+        __syncwarp();
+        if (lane == 0) {
+            s_member = m;
+            sa.out = STAGE == 1 ? members[m].a1 : STAGE == 2 ? members[m].a2 : members[m].phi;
         }
     }
+    __syncthreads();
+    const int m = s_member;
+    const int f44 = members[m].f44;
+    if (REINI && f44 <= q) return;
+    const bool volume = STAGE == 3 && (REINI ? q == f44 - 1 : f44 == 0);
+    const long long lt = t - tile0[m];
+    const int ntx = (sa.L.nx + C::TX - 1) / C::TX, nty = (sa.L.ny + C::TY - 1) / C::TY;
+    const int bx = (int)(lt % ntx);
+    const int by = (int)((lt / ntx) % nty);
+    const int bz = (int)(lt / ((long long)ntx * nty));
+    // the item's arguments in a thread-local copy: the plane loop reads them
+    // across barriers, after which shared memory would be reread
+    const TileArgs a = sa;
+    tile_item<C, REINI, STAGE, ISO>(maps + 3 * m + (STAGE - 1), a, bx, by, bz, volume, smem_raw, red_a, red_b,
+                                    vol_part + 2 * t);
 }
 
 // Face maxima over the cells of one item (x faces 0..nx-2, y 0..ny-2, z
@@ -923,11 +896,10 @@ void launch_stage_cfg(const CUtensorMap& map, const TileArgs& a, bool reini, int
 
 template <class C, bool ISO>
 void launch_batch_cfg(const TiledMember* members, const CUtensorMap* maps, const long long* tile0, int nm,
-                      bool reini, int stage, int q, double* vol_part, unsigned* work, unsigned grid,
-                      cudaStream_t st) {
+                      bool reini, int stage, int q, double* vol_part, unsigned grid, cudaStream_t st) {
     const size_t sm = C::smem();
     const dim3 g(grid), block(C::NT);
-#define R3D_BT(R, S) batch_tile_kernel<C, R, S, ISO><<<g, block, sm, st>>>(members, maps, tile0, nm, q, vol_part, work)
+#define R3D_BT(R, S) batch_tile_kernel<C, R, S, ISO><<<g, block, sm, st>>>(members, maps, tile0, nm, q, vol_part)
     if (reini) {
         if (stage == 1) R3D_BT(true, 1);
         else if (stage == 2) R3D_BT(true, 2);
@@ -1026,10 +998,10 @@ long long tile_items_of(const Layout& L, int kc, int cfg) {
 }
 
 int launch_batch_tile_stage(const TiledMember* members, const CUtensorMap* maps, const long long* tile0, int nm,
-                            int cfg, bool iso, bool reini, int stage, int q, double* vol_part, unsigned* work,
+                            int cfg, bool iso, bool reini, int stage, int q, double* vol_part,
                             unsigned grid, cudaStream_t st) {
     tile_prepare();  // a failure here makes the launch below fail, which the caller reports
-#define R3D_BATCH(C, I) launch_batch_cfg<C, I>(members, maps, tile0, nm, reini, stage, q, vol_part, work, grid, st)
+#define R3D_BATCH(C, I) launch_batch_cfg<C, I>(members, maps, tile0, nm, reini, stage, q, vol_part, grid, st)
     switch (cfg) {
 #define R3D_CFG_CASE(id, tx, ty, ry, ring, minb) \
     case id: if (iso) R3D_BATCH(Cfg##id, true); else R3D_BATCH(Cfg##id, false); break;

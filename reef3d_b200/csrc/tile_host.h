@@ -68,14 +68,12 @@ bool tile_prepare();
 // CTAs per SM configuration `cfg` is built to co-reside (persistent grids)
 int tile_ctas_per_sm(int cfg);
 long long tile_items_of(const Layout& L, int kc, int cfg);
-// Batched persistent tiled stage over the items of nm tiled members, whose
-// maps were encoded for configuration `cfg`.
-// work: two zero-initialised counters the launch takes items from (it leaves
-// them at zero for the next launch on the same stream).
+// Batched tiled stage over the `grid` items of nm tiled members, whose maps
+// were encoded for configuration `cfg`.
 // iso: every member's spacing constants satisfy tile_args_iso.
 int launch_batch_tile_stage(const TiledMember* members, const CUtensorMap* maps, const long long* tile0, int nm,
-                            int cfg, bool iso, bool reini, int stage, int q, double* vol_part, unsigned* work,
-                            unsigned grid, cudaStream_t st);
+                            int cfg, bool iso, bool reini, int stage, int q, double* vol_part, unsigned grid,
+                            cudaStream_t st);
 // Per-item face maxima of the tiled members (3 doubles per item).
 int launch_batch_tile_vmax(const TiledMember* members, const long long* tile0, int nm, int cfg, double* vmax_part,
                            unsigned grid, cudaStream_t st);
