@@ -8,9 +8,11 @@
 namespace r3d {
 namespace f32c {
 
-__device__ __forceinline__ void load7(const float* __restrict__ f, long long c, long long s, float* o) {
+// plain loads: the stage that writes f may still drain when the kernel is
+// launched (launch_step)
+__device__ __forceinline__ void load7(const float* f, long long c, long long s, float* o) {
 #pragma unroll
-    for (int m = 0; m < 7; ++m) o[m] = __ldg(f + c + (m - 3) * s);
+    for (int m = 0; m < 7; ++m) o[m] = f[c + (m - 3) * s];
 }
 
 // Direct-forcing divided difference of the X45 stencils
@@ -39,8 +41,7 @@ __device__ __forceinline__ float df_q32(int x45, double thr, float fa, float fb,
 // arithmetic runs in FP64 on the FP32 values and tables and is rounded to
 // FP32.
 __device__ __forceinline__ float deriv_tables_df6(const float* fv, const double* hv, bool plus,
-                                                  const float* __restrict__ dp, const float* __restrict__ qf,
-                                                  const float* __restrict__ cf, const float* __restrict__ isf, int t) {
+                                                  const float* __restrict__ dp, const float* __restrict__ wt, int t) {
     const int off = plus ? 1 : 0;
     float q[5];
     bool masked[5];
@@ -50,15 +51,14 @@ __device__ __forceinline__ float deriv_tables_df6(const float* fv, const double*
         masked[m - 1] = !(hv[b] < 0.5 && hv[a] < 0.5);
         q[m - 1] = masked[m - 1] ? 0.0f : __fdividef(fv[b] - fv[a], __ldg(dp + t - 4 + m + off));
     }
-    const int side = plus ? 1 : 0;
-    const float* Q = qf + t * 12 + side * 6;
-    const float* C = cf + t * 6 + side * 3;
-    const float* S = isf + t * 18 + side * 9;
+    const float* Q = wt + 18 * (2 * t + off);
+    const float* C = Q + 6;
+    const float* S = Q + 9;
     const bool z1 = masked[2] || masked[3] || masked[4];  // stencil (q3, q4, q5)
     const bool z2 = masked[1] || masked[2] || masked[3];  // (q2, q3, q4)
     const bool z3 = masked[0] || masked[1] || masked[2];  // (q1, q2, q3)
     if (!(z1 && z2 && z3)) {
-        const float r = f32::weno5_tables(Q, C, S, plus, q[0], q[1], q[2], q[3], q[4], z1, z2, z3);
+        const float r = f32::weno5_tables<true>(Q, plus, q[0], q[1], q[2], q[3], q[4], z1, z2, z3);
         if (isfinite(r)) return r;
     }
     // the reference's weighting (src/weno_nug_func.h:48-73, 133-153) in FP64
@@ -94,8 +94,7 @@ __device__ __forceinline__ float deriv_tables_df6(const float* fv, const double*
 // (m-1, m) of the six upwind points, the X45 4 weight at the pair's
 // upwind-most cell.
 __device__ __forceinline__ float deriv_tables_df(const float* fv, const double* hv, bool plus,
-                                                 const float* __restrict__ dp, const float* __restrict__ qf,
-                                                 const float* __restrict__ cf, const float* __restrict__ isf, int t,
+                                                 const float* __restrict__ dp, const float* __restrict__ wt, int t,
                                                  int x45, double thr) {
     const int off = plus ? 1 : 0;
     float q[5];
@@ -104,9 +103,7 @@ __device__ __forceinline__ float deriv_tables_df(const float* fv, const double* 
         const int a = m - 1 + off, b = m + off;
         q[m - 1] = df_q32(x45, thr, fv[a], fv[b], hv[a], hv[b], plus ? hv[b] : hv[a], __ldg(dp + t - 4 + m + off));
     }
-    const int side = plus ? 1 : 0;
-    return f32::weno5_tables(qf + t * 12 + side * 6, cf + t * 6 + side * 3, isf + t * 18 + side * 9, plus, q[0], q[1],
-                             q[2], q[3], q[4]);
+    return f32::weno5_tables(wt + 18 * (2 * t + off), plus, q[0], q[1], q[2], q[3], q[4]);
 }
 
 __device__ __forceinline__ void load7d(const double* __restrict__ f, long long c, long long s, double* o) {
@@ -116,7 +113,7 @@ __device__ __forceinline__ void load7d(const double* __restrict__ f, long long c
 
 // DF: the direct-forcing stencils of g.x45 over g.body (table form).
 template <bool TWO_D, bool UNIFORM, bool DF = false>
-__device__ __forceinline__ float conv_L(const KGrid<float>& g, const float* __restrict__ f,
+__device__ __forceinline__ float conv_L(const KGrid<float>& g, const float* f,
                                         const float* __restrict__ u, const float* __restrict__ v,
                                         const float* __restrict__ w, long long c, int i, int j, int k, float vs) {
     const long long sy = g.L.sy, sz = g.L.sz;
@@ -127,11 +124,11 @@ __device__ __forceinline__ float conv_L(const KGrid<float>& g, const float* __re
     auto axis = [&](long long s, int a, int t, bool plus) {
         if (DF) {
             load7d(g.body, c, s, hv);
-            if (g.x45 == 6) return deriv_tables_df6(fv, hv, plus, g.dxp[a], g.qf[a], g.cf[a], g.isf[a], t);
-            return deriv_tables_df(fv, hv, plus, g.dxp[a], g.qf[a], g.cf[a], g.isf[a], t, g.x45, g.df_thr);
+            if (g.x45 == 6) return deriv_tables_df6(fv, hv, plus, g.dxp[a], g.wt[a], t);
+            return deriv_tables_df(fv, hv, plus, g.dxp[a], g.wt[a], t, g.x45, g.df_thr);
         }
         return UNIFORM ? f32::deriv_uniform<float>(fv, plus, g.rh[a], g.eps_u * g.h[a] * g.h[a])
-                       : f32::deriv_tables(fv, plus, g.dxp[a], g.qf[a], g.cf[a], g.isf[a], t);
+                       : f32::deriv_tables(fv, plus, g.dpr[a], g.wt[a], t);
     };
     float l = 0.0f;
     if (ia != 0.0f) {
@@ -165,15 +162,13 @@ __device__ __forceinline__ float reini_tables(const KGrid<float>& g, const float
     for (int a = 0; a < 3; ++a) {
         if (TWO_D && a == 1) continue;
         const float* f = fa[a];
-        const float xmin = __fdividef(lsv - f[2], __ldg(g.dxp[a] + t[a] - 1));
-        const float xplus = __fdividef(f[4] - lsv, __ldg(g.dxp[a] + t[a]));
-        float d = 0.0f;
-        if (xmin * lsSig > 0.0f && xplus * lsSig > -xmin * lsSig)
-            d = f32::deriv_tables(f, false, g.dxp[a], g.qf[a], g.cf[a], g.isf[a], t[a]);
-        if (xplus * lsSig < 0.0f && xmin * lsSig < -xplus * lsSig)
-            d = f32::deriv_tables(f, true, g.dxp[a], g.qf[a], g.cf[a], g.isf[a], t[a]);
-        if (xplus * lsSig > 0.0f && xmin * lsSig < 0.0f) d = 0.0f;
-        gsum += d * d;
+        const float xmin = (lsv - f[2]) * __ldg(g.dpr[a] + 2 * (t[a] - 1) + 1);
+        const float xplus = (f[4] - lsv) * __ldg(g.dpr[a] + 2 * t[a] + 1);
+        // minus side, plus side, or neither; one evaluation for both sides
+        const bool c1 = xmin * lsSig > 0.0f && xplus * lsSig > -xmin * lsSig;
+        const bool c2 = xplus * lsSig < 0.0f && xmin * lsSig < -xplus * lsSig;
+        const float d = f32::deriv_tables(f, c2, g.dpr[a], g.wt[a], t[a]);
+        gsum += c1 || c2 ? d * d : 0.0f;
     }
     const float dnorm = sqrtf(gsum);
     const float deltax = TWO_D ? 0.5f * (__ldg(g.dxn[0] + t[0]) + __ldg(g.dxn[2] + t[2]))
@@ -184,7 +179,7 @@ __device__ __forceinline__ float reini_tables(const KGrid<float>& g, const float
 }
 
 template <bool TWO_D, bool UNIFORM>
-__device__ __forceinline__ float reini_L(const KGrid<float>& g, const float* __restrict__ f, long long c, int i,
+__device__ __forceinline__ float reini_L(const KGrid<float>& g, const float* f, long long c, int i,
                                          int j, int k) {
     float fx[7], fy[7], fz[7];
     load7(f, c, 1, fx);

@@ -60,35 +60,80 @@ __device__ __forceinline__ R weno5_uniform(bool plus, R d1, R d2, R d3, R d4, R 
     return (al1 * p1 + al2 * p2 + al3 * p3) * inv;
 }
 
-// The reference's non-uniform form (tables, divided differences) in FP32.
-// zero1..zero3: the weight of stencil (q3,q4,q5) / (q2,q3,q4) / (q1,q2,q3)
-// is set to 0 (the X45 = 6 masked differences; at least one stays on).
-__device__ __forceinline__ float weno5_tables(const float* __restrict__ Q, const float* __restrict__ C,
-                                              const float* __restrict__ S, bool plus, float q1, float q2,
-                                              float q3, float q4, float q5, bool zero1 = false,
-                                              bool zero2 = false, bool zero3 = false) {
-    const float dq12 = q1 - q2, dq23 = q2 - q3, dq32 = q3 - q2;
-    const float dq34 = q3 - q4, dq43 = q4 - q3, dq54 = q5 - q4;
-    const float is1 = __ldg(S + 0) * dq54 * dq54 + __ldg(S + 1) * dq54 * dq34 + __ldg(S + 2) * dq34 * dq34;
-    const float is2 = __ldg(S + 3) * dq23 * dq23 + __ldg(S + 4) * dq43 * dq23 + __ldg(S + 5) * dq43 * dq43;
-    const float is3 = __ldg(S + 6) * dq12 * dq12 + __ldg(S + 7) * dq32 * dq12 + __ldg(S + 8) * dq32 * dq32;
-    const float r1 = __frcp_rn(is1 + 1.0e-6f), r2 = __frcp_rn(is2 + 1.0e-6f), r3 = __frcp_rn(is3 + 1.0e-6f);
-    float al1 = __ldg(C + 0) * r1 * r1, al2 = __ldg(C + 1) * r2 * r2, al3 = __ldg(C + 2) * r3 * r3;
-    if (zero1) al1 = 0.0f;
-    if (zero2) al2 = 0.0f;
-    if (zero3) al3 = 0.0f;
-    const float inv = __frcp_rn(al1 + al2 + al3);
-    float p1, p2, p3;
-    if (!plus) {
-        p1 = q4 + __ldg(Q + 0) * (q3 - q4) - __ldg(Q + 1) * (q5 - q4);
-        p2 = q3 + __ldg(Q + 2) * (q4 - q3) - __ldg(Q + 3) * (q2 - q3);
-        p3 = q2 + __ldg(Q + 4) * (q1 - q2) + __ldg(Q + 5) * (q3 - q2);
-    } else {
-        p1 = q4 + __ldg(Q + 0) * (q3 - q4) + __ldg(Q + 1) * (q5 - q4);
-        p2 = q3 + __ldg(Q + 2) * (q2 - q3) - __ldg(Q + 3) * (q4 - q3);
-        p3 = q2 + __ldg(Q + 4) * (q3 - q2) - __ldg(Q + 5) * (q1 - q2);
+__device__ __forceinline__ float rcp_fast(float x) {  // 1 ulp
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// The reference's non-uniform form (tables, divided differences) in FP32,
+// node tables of one (index, side) in the record W = Q0..Q5, C0..C2, S0..S8
+// (8-byte aligned).  The weights c_r / s_r^2 over their sum are formed as
+// c_r (m / s_r)^2 with m the smallest s_r, which stays in the FP32 range
+// whatever the others are (an indicator that overflows has weight 0).  Four
+// approximate reciprocals and no branch on the side, where four rounded ones,
+// five quotients and both sides' code made a stretched 160 x 128 x 96 grid
+// wait for them: see the stage kernels' figures in kernels_f32.cu.
+// MASKS: the weight of stencil (q3,q4,q5) / (q2,q3,q4) / (q1,q2,q3) is 0 where
+// zero1..zero3 (the X45 = 6 masked differences; at least one stays on), and
+// the unscaled c_r / s_r^2 leave the FP32 range (no finite result) where the
+// caller is to evaluate in FP64.
+template <bool MASKS = false>
+__device__ __forceinline__ float weno5_tables(const float* __restrict__ W, bool plus, float q1, float q2, float q3,
+                                              float q4, float q5, bool zero1 = false, bool zero2 = false,
+                                              bool zero3 = false) {
+    float w[18];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) {
+        const float2 v = __ldg(reinterpret_cast<const float2*>(W) + m);
+        w[2 * m] = v.x;
+        w[2 * m + 1] = v.y;
     }
-    return (al1 * p1 + al2 * p2 + al3 * p3) * inv;
+    const float *Q = w, *C = w + 6, *S = w + 9;
+    const float dq12 = q1 - q2, dq23 = q2 - q3, dq34 = q3 - q4, dq54 = q5 - q4;
+    const float s1 = (S[0] * dq54 + S[1] * dq34) * dq54 + S[2] * dq34 * dq34 + 1.0e-6f;
+    const float s2 = (S[3] * dq23 - S[4] * dq34) * dq23 + S[5] * dq34 * dq34 + 1.0e-6f;
+    const float s3 = (S[6] * dq12 - S[7] * dq23) * dq12 + S[8] * dq23 * dq23 + 1.0e-6f;
+    float n1, n2, n3;
+    if (MASKS) {
+        const float r1 = __frcp_rn(s1), r2 = __frcp_rn(s2), r3 = __frcp_rn(s3);
+        n1 = zero1 ? 0.0f : C[0] * r1 * r1;
+        n2 = zero2 ? 0.0f : C[1] * r2 * r2;
+        n3 = zero3 ? 0.0f : C[2] * r3 * r3;
+    } else {
+        const float m = fminf(s1, fminf(s2, s3));
+        const float u1 = m * rcp_fast(s1), u2 = m * rcp_fast(s2), u3 = m * rcp_fast(s3);
+        n1 = C[0] * u1 * u1;
+        n2 = C[1] * u2 * u2;
+        n3 = C[2] * u3 * u3;
+    }
+    const float inv = MASKS ? __frcp_rn(n1 + n2 + n3) : rcp_fast(n1 + n2 + n3);
+    const float t1 = Q[1] * (q5 - q4);
+    const float x2 = plus ? dq23 : -dq34, y2 = plus ? -dq34 : dq23;
+    const float x3 = plus ? -dq23 : dq12, y3 = plus ? dq12 : -dq23;
+    const float t3 = Q[5] * y3;
+    const float p1 = q4 + Q[0] * dq34 + (plus ? t1 : -t1);
+    const float p2 = q3 + Q[2] * x2 - Q[3] * y2;
+    const float p3 = q2 + Q[4] * x3 + (plus ? -t3 : t3);
+    return (n1 * p1 + n2 * p2 + n3 * p3) * inv;
+}
+
+// The uniform form in FP32 from the upwind set d1..d5 (the plus side passes
+// the mirrored set), weights as in weno5_tables; eps = 1e-6 h^2.  Returns h
+// times the derivative.
+__device__ __forceinline__ float weno5_mirrored(float d1, float d2, float d3, float d4, float d5, float eps) {
+    const float a1 = d3 - d4, b1 = d5 - d4, b2 = d2 - d3, b3 = d1 - d2;
+    const float k10 = 10.0f / 3.0f, k11 = 11.0f / 3.0f, k5 = 5.0f / 3.0f, k4 = 4.0f / 3.0f;
+    const float s1 = (k10 * a1 + k11 * b1) * a1 + (k4 * b1 * b1 + eps);
+    const float s2 = (k4 * a1 - k5 * b2) * a1 + (k4 * b2 * b2 + eps);
+    const float s3 = (k10 * b2 - k11 * b3) * b2 + (k4 * b3 * b3 + eps);
+    const float m = fminf(s1, fminf(s2, s3));
+    const float u1 = m * rcp_fast(s1), u2 = m * rcp_fast(s2), u3 = m * rcp_fast(s3);
+    const float n1 = 0.3f * u1 * u1, n2 = 0.6f * u2 * u2, n3 = 0.1f * u3 * u3;
+    const float p1 = d4 + (1.0f / 3.0f) * a1 - (1.0f / 6.0f) * b1;
+    const float p2 = d3 - (1.0f / 3.0f) * a1 - (1.0f / 6.0f) * b2;
+    const float p3 = d2 + (1.0f / 3.0f) * b3 - (11.0f / 6.0f) * b2;
+    return (n1 * p1 + n2 * p2 + n3 * p3) * rcp_fast(n1 + n2 + n3);
 }
 
 // Derivative along an axis from the 7 values f[-3..3] around the cell.
@@ -103,26 +148,23 @@ __device__ __forceinline__ R deriv_uniform(const R* fv, bool plus, R rh, R eps) 
                                  fv[6] - fv[5], eps);
 }
 
-__device__ __forceinline__ float deriv_tables(const float* fv, bool plus, const float* __restrict__ dp,
-                                              const float* __restrict__ qf, const float* __restrict__ cf,
-                                              const float* __restrict__ isf, int t) {
-    float q1, q2, q3, q4, q5;
-    if (!plus) {
-        q1 = __fdividef(fv[1] - fv[0], __ldg(dp + t - 3));
-        q2 = __fdividef(fv[2] - fv[1], __ldg(dp + t - 2));
-        q3 = __fdividef(fv[3] - fv[2], __ldg(dp + t - 1));
-        q4 = __fdividef(fv[4] - fv[3], __ldg(dp + t));
-        q5 = __fdividef(fv[5] - fv[4], __ldg(dp + t + 1));
-    } else {
-        q1 = __fdividef(fv[2] - fv[1], __ldg(dp + t - 2));
-        q2 = __fdividef(fv[3] - fv[2], __ldg(dp + t - 1));
-        q3 = __fdividef(fv[4] - fv[3], __ldg(dp + t));
-        q4 = __fdividef(fv[5] - fv[4], __ldg(dp + t + 1));
-        q5 = __fdividef(fv[6] - fv[5], __ldg(dp + t + 2));
-    }
-    const int side = plus ? 1 : 0;
-    return weno5_tables(qf + t * 12 + side * 6, cf + t * 6 + side * 3, isf + t * 18 + side * 9, plus, q1, q2, q3,
-                        q4, q5);
+template <>
+__device__ __forceinline__ float deriv_uniform<float>(const float* fv, bool plus, float rh, float eps) {
+    float D[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) D[m] = fv[m + 1] - fv[m];
+    return rh * weno5_mirrored(plus ? D[5] : D[0], plus ? D[4] : D[1], plus ? D[3] : D[2], plus ? D[2] : D[3],
+                               plus ? D[1] : D[4], eps);
+}
+
+// dpr: the (DXP, 1/DXP) pairs, wt: the node records, of the axis.
+__device__ __forceinline__ float deriv_tables(const float* fv, bool plus, const float* __restrict__ dpr,
+                                              const float* __restrict__ wt, int t) {
+    float q[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) q[m] = (fv[m + 1] - fv[m]) * __ldg(dpr + 2 * (t + m - 3) + 1);
+    return weno5_tables(wt + 18 * (2 * t + (plus ? 1 : 0)), plus, plus ? q[1] : q[0], plus ? q[2] : q[1],
+                        plus ? q[3] : q[2], plus ? q[4] : q[3], plus ? q[5] : q[4]);
 }
 
 // Reinitialisation right-hand side from the axis stencils (7 values per
@@ -142,11 +184,11 @@ __device__ __forceinline__ R reini_rhs_uniform(const R* fx, const R* fy, const R
         const R* f = fa[a];
         const R xmin = (lsv - f[2]) * rh[a];
         const R xplus = (f[4] - lsv) * rh[a];
-        R d = R(0);
-        if (xmin * lsSig > R(0) && xplus * lsSig > -xmin * lsSig) d = deriv_uniform<R>(f, false, rh[a], eps * hh[a]);
-        if (xplus * lsSig < R(0) && xmin * lsSig < -xplus * lsSig) d = deriv_uniform<R>(f, true, rh[a], eps * hh[a]);
-        if (xplus * lsSig > R(0) && xmin * lsSig < R(0)) d = R(0);
-        g[a] = d;
+        // minus side, plus side, or neither; one evaluation for both sides
+        const bool c1 = xmin * lsSig > R(0) && xplus * lsSig > -xmin * lsSig;
+        const bool c2 = xplus * lsSig < R(0) && xmin * lsSig < -xplus * lsSig;
+        const R d = deriv_uniform<R>(f, c2, rh[a], eps * hh[a]);
+        g[a] = c1 || c2 ? d : R(0);
     }
     const R dnorm = sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
     R sign = lsv * rsqrt_r(lsv * lsv + dnorm * dnorm * deltax * deltax);
