@@ -290,7 +290,7 @@ long long stage_launch(r3d_handle* h, bool reini, int s, bool vol) {
     long long n = stage_launch_plain(h, reini, s, vol);
     if (reini) return n;
     void* out = h->field[s == 1 ? R3D_WORK1 : s == 2 ? R3D_WORK2 : R3D_PHI];
-    if (h->relax) n += launch_relax(h->L, out, fp32(h), relax_zones(h), h->stream);
+    if (h->relax) n += launch_relax(h->L, out, fp32(h), relax_zones(h), h->S.pdl, h->stream);
     if (h->sf_ops) n += launch_solid_forcing(out, fp32(h), h->sf_ops, h->sf_levels, h->stream);
     return n;
 }
@@ -351,7 +351,7 @@ long long picard_correct(r3d_handle* h) {
 long long io_hooks(r3d_handle* h, bool step) {
     if (!h->io) return 0;
     return launch_io_hooks(h->L, h->field[R3D_PHI], h->field[R3D_WORK1], h->field[R3D_WORK2], fp32(h), h->iop,
-                           step, h->stream);
+                           step, h->S.pdl, h->stream);
 }
 
 long long enqueue_reinit(r3d_handle* h, int iters, bool fuse_volume) {
@@ -481,6 +481,7 @@ int r3d_create(const r3d_grid_desc* desc, r3d_handle** out) {
         return bail(R3D_ENOMEM, "scratch allocation failed");
     }
     h->S.npartial = np;
+    h->S.pdl = true;
     h->S.dt = reinterpret_cast<double*>(reinterpret_cast<char*>(h->S.vmax) + 64);
     h->S.vol = reinterpret_cast<double*>(reinterpret_cast<char*>(h->S.vmax) + 128);
     h->S.t = reinterpret_cast<double*>(reinterpret_cast<char*>(h->S.vmax) + 160);
@@ -540,7 +541,9 @@ int r3d_download(r3d_handle* h, int field, double* host, int layout) {
     DeviceGuard dg(h->device, h->batch_stream);
     if (int rc = ensure_staging(h)) return rc;
     const size_t n = host_count(h, layout);
-    if (layout == R3D_LAYOUT_REEF3D) R3D_CUDA(h, cudaMemsetAsync(h->staging, 0, n * sizeof(double), h->stream));
+    // the export writes every cell of a 3D field's padded box (2D: not the y ghost planes)
+    if (layout == R3D_LAYOUT_REEF3D && h->L.two_d)
+        R3D_CUDA(h, cudaMemsetAsync(h->staging, 0, n * sizeof(double), h->stream));
     h->launches += launch_export(h->L, h->field[field], field_fp32(h, field), layout, h->staging, h->stream);
     R3D_CUDA(h, cudaGetLastError());
     R3D_CUDA(h, cudaMemcpyAsync(host, h->staging, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -1833,7 +1836,10 @@ int r3d_domain_create(const r3d_grid_desc* desc, int nslabs, const int* devices,
             break;
         }
         rc = r3d_create(&sd, &h);
-        if (h) h->domain_slab = true;
+        if (h) {
+            h->domain_slab = true;
+            h->S.pdl = false;
+        }
         if (!rc) rc = r3d_set_halo(h, k > 0 ? 1 : 0, k + n < desc->nz ? 1 : 0);
         if (!rc) rc = r3d_set_grid_spacing(h, out4[0], out4[1], out4[2]);
         if (h) {

@@ -1,6 +1,8 @@
 // Kernels shared by both arithmetic forms: host-layout import/export, the
 // standalone wall ghost fill, the FP64 CFL reduction and time step, and the
 // deterministic second pass of the FP64 volume integral.
+#include <type_traits>
+
 #include "r3d_internal.h"
 
 namespace r3d {
@@ -186,6 +188,8 @@ __global__ void __launch_bounds__(256) vmax_f32_kernel(Layout L, const float* __
 // step finds new ones; v keeps its own).
 __global__ void dt_kernel(unsigned long long* vm, const double* vscale, double dxmin, double n47, double* dt,
                           bool reset) {
+    step_next();
+    step_wait();
     // max |s*u| = |s| * max |u| exactly: rounding is monotone
     const double sc = fabs(*vscale);
     const double umax = sc * __longlong_as_double((long long)vm[0]);
@@ -202,6 +206,8 @@ __global__ void dt_kernel(unsigned long long* vm, const double* vscale, double d
 // Second pass: one block sums the per-block partials in a fixed order.
 __global__ void volume_reduce_kernel(const double* __restrict__ partial, long long n, double* out, double* t,
                                      double* vscale, const double* dt, double period) {
+    step_next();
+    step_wait();
     __shared__ double sa[1024], sb[1024];
     double a = 0.0, b = 0.0;
     for (long long t = threadIdx.x; t < n; t += blockDim.x) {
@@ -359,10 +365,14 @@ __global__ void __launch_bounds__(256) airy_kernel(Layout L, T* __restrict__ u, 
 // (gcval 1: a Neumann copy into the three layers, src/gc_epol4.cpp:90-93,
 // src/gc_neumann.cpp:29-54; 2D skips y), and the volume partials of
 // volume_direct_kernel.
-template <typename T>
+template <typename T, bool STEP>
 __global__ void fluid_kernel(Layout L, const T* __restrict__ phi, T* __restrict__ ro, T* __restrict__ visc,
                              const double* __restrict__ dxn, const double* __restrict__ dyn,
                              const double* __restrict__ dzn, double psi, FluidConst fc, double* partial) {
+    if (STEP) {
+        step_next();
+        step_wait();
+    }
     const double PI_REF = 3.14159265359;  // src/definitions.h:37
     const int j = blockIdx.y, k = blockIdx.z;
     double a = 0.0, b = 0.0;
@@ -644,6 +654,8 @@ __device__ void io_levels(const In& in, const Out& out, const IoParams& p) {
 
 template <typename T>
 __global__ void __launch_bounds__(kIoThreads) io_level_kernel(Layout L, const T* __restrict__ phi, IoParams p) {
+    step_next();
+    step_wait();
     io_levels(CellHeights<T>{L, phi, p, -1}, CellHeights<T>{L, phi, p, L.nx - 1}, p);
 }
 
@@ -678,6 +690,8 @@ __global__ void __launch_bounds__(kIoThreads) io_fold_kernel(const double* __res
 template <typename T>
 __global__ void __launch_bounds__(256) io_ghost_kernel(Layout L, T* __restrict__ phi, T* __restrict__ a1,
                                                        T* __restrict__ a2, IoParams p, int step) {
+    step_next();
+    step_wait();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= L.ny * L.nz) return;
     const int j = e / L.nz, k = e - j * L.nz;
@@ -801,21 +815,21 @@ __global__ void netvol_kernel(double* pic, const double* dt, double qi, double q
 
 }  // namespace
 
-int launch_io_hooks(const Layout& L, void* phi, void* a1, void* a2, bool fp32, const IoParams& p, bool step,
+int launch_io_hooks(const Layout& L, void* phi, void* a1, void* a2, bool fp32, const IoParams& p, bool step, bool pdl,
                     cudaStream_t st) {
     const int rows = L.ny * L.nz;
     const int blocks = (rows + 255) / 256;
     int n = 0;
     if (step && !p.waves) {
-        if (fp32) io_level_kernel<float><<<1, kIoThreads, 0, st>>>(L, static_cast<const float*>(phi), p);
-        else io_level_kernel<double><<<1, kIoThreads, 0, st>>>(L, static_cast<const double*>(phi), p);
+        if (fp32) launch_small(pdl, io_level_kernel<float>, 1, kIoThreads, st, L, static_cast<const float*>(phi), p);
+        else launch_small(pdl, io_level_kernel<double>, 1, kIoThreads, st, L, static_cast<const double*>(phi), p);
         ++n;
     }
     if (fp32)
-        io_ghost_kernel<float><<<blocks, 256, 0, st>>>(L, static_cast<float*>(phi), static_cast<float*>(a1),
+        launch_small(pdl, io_ghost_kernel<float>, blocks, 256, st, L, static_cast<float*>(phi), static_cast<float*>(a1),
                                                        static_cast<float*>(a2), p, step ? 1 : 0);
     else
-        io_ghost_kernel<double><<<blocks, 256, 0, st>>>(L, static_cast<double*>(phi), static_cast<double*>(a1),
+        launch_small(pdl, io_ghost_kernel<double>, blocks, 256, st, L, static_cast<double*>(phi), static_cast<double*>(a1),
                                                         static_cast<double*>(a2), p, step ? 1 : 0);
     return n + 1;
 }
@@ -871,6 +885,8 @@ int launch_vtu_nodes(const Layout& L, const void* phi, const void* ro, const voi
 // ghostcell::start4 afterwards does (src/levelset_RK3.cpp:125-127).
 template <typename T>
 __global__ void relax_kernel(Layout L, T* f, RelaxZones z) {
+    step_next();
+    step_wait();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)z.ncol * L.nz) return;
     const int q = (int)(t / L.nz), k = (int)(t % L.nz);
@@ -898,12 +914,12 @@ __global__ void relax_kernel(Layout L, T* f, RelaxZones z) {
     }
 }
 
-int launch_relax(const Layout& L, void* f, bool fp32, const RelaxZones& z, cudaStream_t st) {
+int launch_relax(const Layout& L, void* f, bool fp32, const RelaxZones& z, bool pdl, cudaStream_t st) {
     const long long n = (long long)z.ncol * L.nz;
     if (n <= 0) return 0;
     const unsigned g = (unsigned)((n + 255) / 256);
-    if (fp32) relax_kernel<float><<<g, 256, 0, st>>>(L, static_cast<float*>(f), z);
-    else relax_kernel<double><<<g, 256, 0, st>>>(L, static_cast<double*>(f), z);
+    if (fp32) launch_small(pdl, relax_kernel<float>, g, 256, st, L, static_cast<float*>(f), z);
+    else launch_small(pdl, relax_kernel<double>, g, 256, st, L, static_cast<double*>(f), z);
     return 1;
 }
 
@@ -1006,15 +1022,17 @@ int launch_fluid_update(const Layout& L, const void* phi, void* ro, void* visc, 
                         const double* dyn, const double* dzn, double psi, const FluidConst& fc, bool clock,
                         double period, const Scratch& s, cudaStream_t st) {
     const dim3 grid(1, L.ny, L.nz), block(256);
-    if (fp32)
-        fluid_kernel<float><<<grid, block, 0, st>>>(L, static_cast<const float*>(phi), static_cast<float*>(ro),
-                                                    static_cast<float*>(visc), dxn, dyn, dzn, psi, fc, s.partial);
-    else
-        fluid_kernel<double><<<grid, block, 0, st>>>(L, static_cast<const double*>(phi), static_cast<double*>(ro),
-                                                     static_cast<double*>(visc), dxn, dyn, dzn, psi, fc, s.partial);
+    auto run = [&](auto* p, auto* r, auto* m) {
+        using T = std::remove_pointer_t<decltype(r)>;
+        if (step_grid(s.pdl, grid))
+            launch_step(fluid_kernel<T, true>, grid, block, st, L, p, r, m, dxn, dyn, dzn, psi, fc, s.partial);
+        else fluid_kernel<T, false><<<grid, block, 0, st>>>(L, p, r, m, dxn, dyn, dzn, psi, fc, s.partial);
+    };
+    if (fp32) run(static_cast<const float*>(phi), static_cast<float*>(ro), static_cast<float*>(visc));
+    else run(static_cast<const double*>(phi), static_cast<double*>(ro), static_cast<double*>(visc));
     if (clock)
-        volume_reduce_kernel<<<1, 1024, 0, st>>>(s.partial, (long long)L.ny * L.nz, s.vol, s.t, s.vscale, s.dt,
-                                                 period);
+        launch_small(s.pdl, volume_reduce_kernel, 1, 1024, st, s.partial, (long long)L.ny * L.nz, s.vol, s.t, s.vscale,
+                    s.dt, period);
     else
         volume_reduce_kernel<<<1, 1024, 0, st>>>(s.partial, (long long)L.ny * L.nz, s.vol, nullptr, nullptr,
                                                  nullptr, 0.0);
@@ -1082,7 +1100,7 @@ int launch_vmax(const Layout& L, const void* u, const void* v, const void* w, bo
 }
 
 int launch_dt(double dxmin, double n47, const Scratch& s, bool reset, cudaStream_t st) {
-    dt_kernel<<<1, 1, 0, st>>>(s.vmax, s.vscale, dxmin, n47, s.dt, reset);
+    launch_small(s.pdl, dt_kernel, 1, 1, st, s.vmax, s.vscale, dxmin, n47, s.dt, reset);
     return 1;
 }
 
@@ -1092,7 +1110,7 @@ int launch_cfl(const Layout& L, const void* u, const void* v, const void* w, boo
 }
 
 int launch_volume_reduce(const Layout&, const Scratch& s, long long nblocks, double period, cudaStream_t st) {
-    volume_reduce_kernel<<<1, 1024, 0, st>>>(s.partial, nblocks, s.vol, s.t, s.vscale, s.dt, period);
+    launch_small(s.pdl, volume_reduce_kernel, 1, 1024, st, s.partial, nblocks, s.vol, s.t, s.vscale, s.dt, period);
     return 1;
 }
 

@@ -44,8 +44,13 @@ __device__ __forceinline__ void block_sum2(double a, double b, double* dst) {
     }
 }
 
-template <bool TWO_D, int STAGE, bool REINI, bool VOLUME, bool UNIFORM, bool DF = false>
+// STEP: launched by launch_step.
+template <bool TWO_D, int STAGE, bool REINI, bool VOLUME, bool UNIFORM, bool DF, bool STEP>
 __global__ void __launch_bounds__(kBX * kBY) stage_kernel32(KGrid<float> g, StageArgs32 a) {
+    if (STEP) {
+        step_next();
+        step_wait();
+    }
     const int i = blockIdx.x * kBX + threadIdx.x;
     const int j = TWO_D ? 0 : blockIdx.y * kBY + threadIdx.y;
     const int k = TWO_D ? blockIdx.z * kBY + threadIdx.y : blockIdx.z;
@@ -64,8 +69,8 @@ __global__ void __launch_bounds__(kBX * kBY) stage_kernel32(KGrid<float> g, Stag
         const float fn = a.fn[c];
         float val;
         if (STAGE == 1) val = fn + dtc * Lc;
-        else if (STAGE == 2) val = 0.75f * fn + 0.25f * (__ldg(a.fs + c) + dtc * Lc);
-        else val = (1.0f / 3.0f) * fn + (2.0f / 3.0f) * (__ldg(a.fs + c) + dtc * Lc);
+        else if (STAGE == 2) val = 0.75f * fn + 0.25f * (a.fs[c] + dtc * Lc);
+        else val = (1.0f / 3.0f) * fn + (2.0f / 3.0f) * (a.fs[c] + dtc * Lc);
         a.out[c] = val;
         // x faces: inflow / outflow faces with ghost label 0 keep their
         // ghosts; an inflow face also gets the edge ghost (-1, j, nz)
@@ -117,9 +122,13 @@ dim3 grid_of32(const Layout& L) {
 }
 
 template <bool TWO_D, bool REINI, bool UNIFORM, bool DF = false>
-void launch_t(const KGrid<float>& g, const StageArgs32& a, int stage, bool volume, cudaStream_t st) {
+void launch_t(const KGrid<float>& g, const StageArgs32& a, int stage, bool volume, bool pdl, cudaStream_t st) {
     const dim3 grid = grid_of32(g.L), block(kBX, kBY);
-#define R3D_L32(S, V) stage_kernel32<TWO_D, S, REINI, V, UNIFORM, DF><<<grid, block, 0, st>>>(g, a)
+#define R3D_L32(S, V)                                                                                               \
+    do {                                                                                                            \
+        if (step_grid(pdl, grid)) launch_step(stage_kernel32<TWO_D, S, REINI, V, UNIFORM, DF, true>, grid, block, st, g, a); \
+        else stage_kernel32<TWO_D, S, REINI, V, UNIFORM, DF, false><<<grid, block, 0, st>>>(g, a);                  \
+    } while (0)
     if (stage == 1) { if (volume) R3D_L32(1, true); else R3D_L32(1, false); }
     else if (stage == 2) { if (volume) R3D_L32(2, true); else R3D_L32(2, false); }
     else { if (volume) R3D_L32(3, true); else R3D_L32(3, false); }
@@ -127,18 +136,19 @@ void launch_t(const KGrid<float>& g, const StageArgs32& a, int stage, bool volum
 }
 
 template <bool REINI>
-void launch_any(const KGrid<float>& g, const StageArgs32& a, int stage, bool volume, bool uniform, cudaStream_t st) {
+void launch_any(const KGrid<float>& g, const StageArgs32& a, int stage, bool volume, bool uniform, bool pdl,
+                cudaStream_t st) {
     if (!REINI && g.x45) {  // direct-forcing stencils (table form)
-        if (g.L.two_d) launch_t<true, false, false, true>(g, a, stage, volume, st);
-        else launch_t<false, false, false, true>(g, a, stage, volume, st);
+        if (g.L.two_d) launch_t<true, false, false, true>(g, a, stage, volume, pdl, st);
+        else launch_t<false, false, false, true>(g, a, stage, volume, pdl, st);
         return;
     }
     if (g.L.two_d) {
-        if (uniform) launch_t<true, REINI, true>(g, a, stage, volume, st);
-        else launch_t<true, REINI, false>(g, a, stage, volume, st);
+        if (uniform) launch_t<true, REINI, true>(g, a, stage, volume, pdl, st);
+        else launch_t<true, REINI, false>(g, a, stage, volume, pdl, st);
     } else {
-        if (uniform) launch_t<false, REINI, true>(g, a, stage, volume, st);
-        else launch_t<false, REINI, false>(g, a, stage, volume, st);
+        if (uniform) launch_t<false, REINI, true>(g, a, stage, volume, pdl, st);
+        else launch_t<false, REINI, false>(g, a, stage, volume, pdl, st);
     }
 }
 
@@ -163,13 +173,13 @@ bool is_uniform(const KGrid<float>& g) { return g.h[0] > 0.0f; }
 
 int launch_conv_stage_f32(const KGrid<float>& g, const Fields& f, int stage, const Scratch& s, bool volume,
                           cudaStream_t st) {
-    launch_any<false>(g, args32(f, stage, s), stage, volume, is_uniform(g), st);
+    launch_any<false>(g, args32(f, stage, s), stage, volume, is_uniform(g), s.pdl, st);
     return 1;
 }
 
 int launch_reini_stage_f32(const KGrid<float>& g, const Fields& f, int stage, const Scratch& s, bool volume,
                            cudaStream_t st) {
-    launch_any<true>(g, args32(f, stage, s), stage, volume, is_uniform(g), st);
+    launch_any<true>(g, args32(f, stage, s), stage, volume, is_uniform(g), s.pdl, st);
     return 1;
 }
 

@@ -103,12 +103,15 @@ __device__ __forceinline__ void heaviside_volume(const KGrid<double>& g, double 
 //   s=3: out = 1/3 fn + 2/3 fs + 2/3 dt L(fs)
 // Reinit stage s of src/reini_RK3.cpp:113-137: the same with the per-cell
 // pseudo time step.
-template <bool TWO_D, int STAGE, bool REINI, bool VOLUME, bool DF = false>
+// STEP: launched by launch_step.
+template <bool TWO_D, int STAGE, bool REINI, bool VOLUME, bool DF, bool STEP>
 __global__ void __launch_bounds__(kBX * kBY, REINI ? kReiniBlocks : kConvBlocks) stage_kernel(KGrid<double> g, StageArgs a) {
+    if (STEP) step_next();
     int i, j, k;
     cell_of_thread(g.L, TWO_D, i, j, k);
     const bool active = i < g.L.nx && j < g.L.ny && k < g.L.nz;
     double v1 = 0.0, v2 = 0.0;
+    if (STEP) step_wait();
     if (active) {
         const long long c = (long long)(k + g.L.gz) * g.L.sz + (long long)(j + g.L.gy) * g.L.sy + (i + g.L.gx);
         double Lc, dtc;
@@ -125,8 +128,8 @@ __global__ void __launch_bounds__(kBX * kBY, REINI ? kReiniBlocks : kConvBlocks)
         const double fn = a.fn[c];
         double val;
         if (STAGE == 1) val = fn + dtc * Lc;
-        else if (STAGE == 2) val = 0.75 * fn + 0.25 * __ldg(a.fs + c) + 0.25 * dtc * Lc;
-        else val = (1.0 / 3.0) * fn + (2.0 / 3.0) * __ldg(a.fs + c) + (2.0 / 3.0) * dtc * Lc;
+        else if (STAGE == 2) val = 0.75 * fn + 0.25 * a.fs[c] + 0.25 * dtc * Lc;
+        else val = (1.0 / 3.0) * fn + (2.0 / 3.0) * a.fs[c] + (2.0 / 3.0) * dtc * Lc;
         a.out[c] = val;
         write_ghosts(g.L, a.out, c, i, j, k, val);
         if (VOLUME) heaviside_volume(g, val, i, j, k, v1, v2);
@@ -161,18 +164,17 @@ dim3 grid_of(const Layout& L) {
 }
 
 template <bool TWO_D, bool REINI, bool DF = false>
-void launch_stage_t(const KGrid<double>& g, const StageArgs& a, int stage, bool volume, cudaStream_t st) {
+void launch_stage_t(const KGrid<double>& g, const StageArgs& a, int stage, bool volume, bool pdl, cudaStream_t st) {
     const dim3 grid = grid_of(g.L), block(kBX, kBY);
-    if (stage == 1) {
-        if (volume) stage_kernel<TWO_D, 1, REINI, true, DF><<<grid, block, 0, st>>>(g, a);
-        else stage_kernel<TWO_D, 1, REINI, false, DF><<<grid, block, 0, st>>>(g, a);
-    } else if (stage == 2) {
-        if (volume) stage_kernel<TWO_D, 2, REINI, true, DF><<<grid, block, 0, st>>>(g, a);
-        else stage_kernel<TWO_D, 2, REINI, false, DF><<<grid, block, 0, st>>>(g, a);
-    } else {
-        if (volume) stage_kernel<TWO_D, 3, REINI, true, DF><<<grid, block, 0, st>>>(g, a);
-        else stage_kernel<TWO_D, 3, REINI, false, DF><<<grid, block, 0, st>>>(g, a);
-    }
+#define R3D_L64(S, V)                                                                                      \
+    do {                                                                                                   \
+        if (step_grid(pdl, grid)) launch_step(stage_kernel<TWO_D, S, REINI, V, DF, true>, grid, block, st, g, a); \
+        else stage_kernel<TWO_D, S, REINI, V, DF, false><<<grid, block, 0, st>>>(g, a);                    \
+    } while (0)
+    if (stage == 1) { if (volume) R3D_L64(1, true); else R3D_L64(1, false); }
+    else if (stage == 2) { if (volume) R3D_L64(2, true); else R3D_L64(2, false); }
+    else { if (volume) R3D_L64(3, true); else R3D_L64(3, false); }
+#undef R3D_L64
 }
 
 StageArgs stage_args(const Fields& f, int stage, const Scratch& s) {
@@ -196,11 +198,11 @@ int launch_conv_stage_f64(const KGrid<double>& g, const Fields& f, int stage, co
                           cudaStream_t st) {
     const StageArgs a = stage_args(f, stage, s);
     if (g.x45) {  // direct-forcing stencils (X45 1..6)
-        if (g.L.two_d) launch_stage_t<true, false, true>(g, a, stage, volume, st);
-        else launch_stage_t<false, false, true>(g, a, stage, volume, st);
+        if (g.L.two_d) launch_stage_t<true, false, true>(g, a, stage, volume, s.pdl, st);
+        else launch_stage_t<false, false, true>(g, a, stage, volume, s.pdl, st);
     } else {
-        if (g.L.two_d) launch_stage_t<true, false>(g, a, stage, volume, st);
-        else launch_stage_t<false, false>(g, a, stage, volume, st);
+        if (g.L.two_d) launch_stage_t<true, false>(g, a, stage, volume, s.pdl, st);
+        else launch_stage_t<false, false>(g, a, stage, volume, s.pdl, st);
     }
     return 1;
 }
@@ -208,8 +210,8 @@ int launch_conv_stage_f64(const KGrid<double>& g, const Fields& f, int stage, co
 int launch_reini_stage_f64(const KGrid<double>& g, const Fields& f, int stage, const Scratch& s, bool volume,
                            cudaStream_t st) {
     const StageArgs a = stage_args(f, stage, s);
-    if (g.L.two_d) launch_stage_t<true, true>(g, a, stage, volume, st);
-    else launch_stage_t<false, true>(g, a, stage, volume, st);
+    if (g.L.two_d) launch_stage_t<true, true>(g, a, stage, volume, s.pdl, st);
+    else launch_stage_t<false, true>(g, a, stage, volume, s.pdl, st);
     return 1;
 }
 

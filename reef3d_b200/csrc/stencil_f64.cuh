@@ -12,6 +12,10 @@
 namespace r3d {
 namespace f64 {
 
+// The level set f is read by plain loads, not through the read-only path: a
+// stage may be launched while the one that writes f still drains
+// (launch_step), so f does not stay unwritten for the kernel's whole life.
+
 // a / b rounded to nearest from r = 1/b rounded to nearest (the IEEE
 // reciprocal, tabulated per grid spacing): q0 = a r, then two residual
 // corrections with fused multiply-adds (P. Markstein, "Computation of
@@ -129,14 +133,14 @@ __device__ __forceinline__ double weno5(const double* __restrict__ W, bool plus,
 // q_m = (f_m - f_{m-1}) / DXP[t+o+m-1], the IEEE quotient formed by div_rn
 // from the reciprocal table rp of dp.  The side is a runtime value, so a
 // warp whose cells take different sides runs one evaluation, not both.
-__device__ __forceinline__ double deriv(const double* __restrict__ f, long long c, long long s,
+__device__ __forceinline__ double deriv(const double* f, long long c, long long s,
                                         const double* __restrict__ dpr, const double* __restrict__ wt, int t,
                                         bool plus) {
     const int o = plus ? -2 : -3;
     const double* p = f + c + o * s;
     const double* d = dpr + 2 * (t + o);
-    const double f0 = __ldg(p), f1 = __ldg(p + s), f2 = __ldg(p + 2 * s);
-    const double f3 = __ldg(p + 3 * s), f4 = __ldg(p + 4 * s), f5 = __ldg(p + 5 * s);
+    const double f0 = p[0], f1 = p[s], f2 = p[2 * s];
+    const double f3 = p[3 * s], f4 = p[4 * s], f5 = p[5 * s];
     const double2 e1 = ldg2(d), e2 = ldg2(d + 2), e3 = ldg2(d + 4), e4 = ldg2(d + 6), e5 = ldg2(d + 8);
     const double q1 = div_rn(f1 - f0, e1.x, e1.y);
     const double q2 = div_rn(f2 - f1, e2.x, e2.y);
@@ -181,7 +185,7 @@ __device__ __forceinline__ double df_q(int x45, double thr, double fa, double fb
 }
 
 // deriv with the direct-forcing differences of df_q.
-__device__ __forceinline__ double deriv_df(const double* __restrict__ f, const double* __restrict__ h, long long c,
+__device__ __forceinline__ double deriv_df(const double* f, const double* __restrict__ h, long long c,
                                            long long s, const double* __restrict__ dp,
                                            const double* __restrict__ wt, int t, bool plus, int x45, double thr) {
     const int o = plus ? -2 : -3;
@@ -190,7 +194,7 @@ __device__ __forceinline__ double deriv_df(const double* __restrict__ f, const d
     double fv[6], hv[6];
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
-        fv[m] = __ldg(f + b0 + m * s);
+        fv[m] = f[b0 + m * s];
         hv[m] = __ldg(h + b0 + m * s);
     }
     double q[5];
@@ -207,7 +211,7 @@ __device__ __forceinline__ double deriv_df(const double* __restrict__ f, const d
 // The stored face velocities are multiplied by vs (1 leaves them exact).
 // DF: the direct-forcing stencils of g.x45 (g.body) replace the plain ones.
 template <bool TWO_D, bool DF = false>
-__device__ __forceinline__ double conv_L(const KGrid<double>& g, const double* __restrict__ f,
+__device__ __forceinline__ double conv_L(const KGrid<double>& g, const double* f,
                                          const double* __restrict__ u, const double* __restrict__ v,
                                          const double* __restrict__ w, long long c, int i, int j, int k,
                                          double vs) {
@@ -239,11 +243,11 @@ __device__ __forceinline__ double conv_L(const KGrid<double>& g, const double* _
 // F49=0 interface test (src/reinidisc_fsf.cpp:70-72).  In 2D the y
 // neighbours are ghost planes the reference never writes (zero).
 template <bool TWO_D>
-__device__ __forceinline__ bool same_sign(const double* __restrict__ f, long long c, long long sy,
+__device__ __forceinline__ bool same_sign(const double* f, long long c, long long sy,
                                           long long sz) {
-    const double f0 = __ldg(f + c), xp = __ldg(f + c + 1), xm = __ldg(f + c - 1);
-    const double yp = TWO_D ? 0.0 : __ldg(f + c + sy), ym = TWO_D ? 0.0 : __ldg(f + c - sy);
-    const double zp = __ldg(f + c + sz), zm = __ldg(f + c - sz);
+    const double f0 = f[c], xp = f[c + 1], xm = f[c - 1];
+    const double yp = TWO_D ? 0.0 : f[c + sy], ym = TWO_D ? 0.0 : f[c - sy];
+    const double zp = f[c + sz], zm = f[c - sz];
     return (f0 >= 0.0 && xp >= 0.0 && xm >= 0.0 && yp >= 0.0 && ym >= 0.0 && zp >= 0.0 && zm >= 0.0) ||
            (f0 < 0.0 && xp < 0.0 && xm < 0.0 && yp < 0.0 && ym < 0.0 && zp < 0.0 && zm < 0.0);
 }
@@ -254,11 +258,11 @@ __device__ __forceinline__ bool same_sign(const double* __restrict__ f, long lon
 // reads.  Each is the quotient deriv forms for that face, and faces 2 and 3
 // are the backward and forward differences of the reinitialisation's
 // Godunov test.
-__device__ __forceinline__ void faces6(const double* __restrict__ f, long long c, long long s,
+__device__ __forceinline__ void faces6(const double* f, long long c, long long s,
                                        const double* __restrict__ dpr, int t, double* Q) {
     double fv[7];
 #pragma unroll
-    for (int m = 0; m < 7; ++m) fv[m] = __ldg(f + c + (m - 3) * s);
+    for (int m = 0; m < 7; ++m) fv[m] = f[c + (m - 3) * s];
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
         const double2 e = ldg2(dpr + 2 * (t + m - 3));
@@ -287,12 +291,12 @@ __device__ __forceinline__ double reini_axis(const double* Q, double lsSig, cons
 // stencil (the reference divides the two Godunov faces a second time; the
 // quotients are the same).
 template <bool TWO_D>
-__device__ __forceinline__ double reini_L(const KGrid<double>& g, const double* __restrict__ f, long long c,
+__device__ __forceinline__ double reini_L(const KGrid<double>& g, const double* f, long long c,
                                           int i, int j, int k) {
     const long long sy = g.L.sy, sz = g.L.sz;
     const int ti = i + 5, tj = j + 5, tk = k + 5;
     double dx = 0.0, dy = 0.0, dz = 0.0;
-    const double lsv = __ldg(f + c);
+    const double lsv = f[c];
     // lsv / sqrt(lsv * lsv): the square root of a correctly rounded square
     // is |lsv| exactly (binary arithmetic, round to nearest, no overflow), so
     // the quotient is the sign; the formula itself where the square overflows
