@@ -343,14 +343,16 @@ __global__ void __launch_bounds__(256) airy_kernel(Layout L, T* __restrict__ u, 
             mu = fmax(mu, __shfl_down_sync(0xffffffffu, mu, o));
             mw = fmax(mw, __shfl_down_sync(0xffffffffu, mw, o));
         }
-        __shared__ double s[2][8];
+        // the warps' maxima take the tables' place (28 values at least): no
+        // shared memory of its own, so both forms have the tables' limits
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        if (lane == 0) { s[0][warp] = mu; s[1][warp] = mw; }
+        __syncthreads();
+        if (lane == 0) { tab[warp] = mu; tab[8 + warp] = mw; }
         __syncthreads();
         if (threadIdx.x == 0) {
             for (int q = 1; q < (int)(blockDim.x >> 5); ++q) {
-                mu = fmax(mu, s[0][q]);
-                mw = fmax(mw, s[1][q]);
+                mu = fmax(mu, tab[q]);
+                mw = fmax(mw, tab[8 + q]);
             }
             atomicMax(vmax + 0, (unsigned long long)__double_as_longlong(mu));
             atomicMax(vmax + 2, (unsigned long long)__double_as_longlong(mw));
@@ -1005,8 +1007,9 @@ int launch_airy(const Layout& L, void* u, void* w, bool fp32, const double* coor
 }
 
 int airy_prepare(const Layout& L) {
+    constexpr int kMost = 227 * 1024;  // of a block; the kernels have no static shared memory
     const size_t smem = airy_smem_bytes(L);
-    if (smem > 227 * 1024) return 1;
+    if (smem > kMost) return 1;
     if (smem > 48 * 1024) {
         auto allow = [&](auto* k) {
             return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;

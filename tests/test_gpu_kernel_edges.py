@@ -177,3 +177,44 @@ def test_pageable_copies(nz, precision):
         m = visible_mask(nx, ny, nz)
         got = ls.download(r3d.U)
         assert np.array_equal(got[m], r[m]) and not np.any(got[~m])
+
+
+def airy_flume(nx, nz, precision):
+    """A thin flume of nx x nz cells, its depth half the height, with a sheet
+    at the still water and the Airy generator on."""
+    nodes = (r3d.uniform_nodes(nx, nx / nz), r3d.uniform_nodes(1, 1.0 / nz), r3d.uniform_nodes(nz))
+    ls = instance((nx, 1, nz), precision, nodes)
+    z = (np.arange(nz) + 0.5) / nz
+    ls.upload(r3d.PHI, np.broadcast_to(0.5 - z[:, None, None], (nz, 1, nx)).copy(), r3d.LAYOUT_DENSE)
+    ls.ghost_fill()
+    ls.set_time(0.0)
+    ls.set_velocity_airy(0.05, 2.0, 0.5)
+    return ls
+
+
+@pytest.mark.parametrize("precision", [r3d.FP32, r3d.FP64])
+@pytest.mark.parametrize("edge", [3052, 3053, 3060, 3061, 14508, 14509, 14516])
+def test_airy_run_at_the_shared_memory_limits(edge, precision):
+    """Adaptive runs of the Airy generator where its tables, 16 (nx + nz + 12)
+    bytes, reach the 48 KB that need no opt-in and the 227 KB of a block: one
+    step (launched) and three (replayed from a graph) are single steps with
+    r3d_cfl_dt before each."""
+    nz = 56
+    a, b = airy_flume(edge - nz, nz, precision), airy_flume(edge - nz, nz, precision)
+    try:
+        for steps in (1, 3):
+            a.run(steps, adaptive=True)
+            for _ in range(steps):
+                b.step(b.cfl_dt())
+            assert a.time() == b.time() > 0.0
+            assert np.array_equal(dense(a), dense(b))
+    finally:
+        a.close()
+        b.close()
+
+
+def test_airy_refused_beyond_shared_memory():
+    """One cell more than the tables' limit is refused when the generator is
+    set, as before it is used."""
+    with pytest.raises(r3d.R3DError):
+        airy_flume(14517 - 56, 56, r3d.FP32).close()
