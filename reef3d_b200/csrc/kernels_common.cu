@@ -1011,8 +1011,10 @@ int airy_prepare(const Layout& L) {
     const size_t smem = airy_smem_bytes(L);
     if (smem > kMost) return 1;
     if (smem > 48 * 1024) {
+        // a kernel's limit holds for every instance: always the most, so that
+        // a short grid set up later does not lower a long one's
         auto allow = [&](auto* k) {
-            return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+            return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost) == cudaSuccess;
         };
         if (!allow(airy_kernel<float, false>) || !allow(airy_kernel<float, true>) ||
             !allow(airy_kernel<double, false>) || !allow(airy_kernel<double, true>))

@@ -218,3 +218,16 @@ def test_airy_refused_beyond_shared_memory():
     set, as before it is used."""
     with pytest.raises(r3d.R3DError):
         airy_flume(14517 - 56, 56, r3d.FP32).close()
+
+
+def test_airy_instances_leave_each_other_their_shared_memory():
+    """A shorter flume set up later does not lower what a longer one's launches
+    may take."""
+    long, short = airy_flume(6000, 56, r3d.FP32), airy_flume(3100, 56, r3d.FP32)
+    try:
+        for ls in (long, short):
+            ls.run(1, adaptive=True)
+            ls.sync()
+    finally:
+        long.close()
+        short.close()
