@@ -428,6 +428,11 @@ int r3d_init_spheres_tg(r3d_handle* h, int nspheres, const double* spheres, int 
  *                 wait for their own copies, return -- and the next
  *                 r3d_sync reports R3D_ETIMEOUT; the instance stays usable.
  *                 Cleared by that step.  No effect off the tiled path.
+ *  R3D_OPT_LAUNCH_TEST  diagnostic for rejected launches: 1 makes the next
+ *                 r3d_cfl_dt, r3d_ls_step or r3d_ls_run begin with a launch
+ *                 that the CUDA runtime refuses (nothing runs on the device),
+ *                 so the call returns R3D_EDEVICE with the level set
+ *                 untouched; the instance stays usable.  Cleared by that call.
  *  R3D_OPT_TILE_CFG  tile configuration of the tiled kernels, 0 ..
  *                 r3d_tile_config_count()-1 (r3d_tile_config_describe: tile
  *                 shape, rows per thread, ring depth); the level set is the
@@ -439,6 +444,7 @@ int r3d_init_spheres_tg(r3d_handle* h, int nspheres, const double* spheres, int 
 #define R3D_OPT_BAND64 2
 #define R3D_OPT_WAIT_TEST 3
 #define R3D_OPT_TILE_CFG 4
+#define R3D_OPT_LAUNCH_TEST 5
 #define R3D_OPT_TILE_CFG_REINIT 6
 #define R3D_OPT_CHUNK_REINIT 7
 int r3d_set_option(r3d_handle* h, int option, int value);

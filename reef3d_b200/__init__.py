@@ -23,7 +23,7 @@ FP64, FP32 = 0, 1
 PHI, U, V, W, L, WORK1, WORK2, RO, VISC, BODY = range(10)
 LAYOUT_REEF3D, LAYOUT_DENSE = 0, 1
 STAGE_CONVECTION, STAGE_REINIT = 0, 1
-OPT_TILED, OPT_CHUNK, OPT_BAND64, OPT_WAIT_TEST, OPT_TILE_CFG = 0, 1, 2, 3, 4
+OPT_TILED, OPT_CHUNK, OPT_BAND64, OPT_WAIT_TEST, OPT_TILE_CFG, OPT_LAUNCH_TEST = 0, 1, 2, 3, 4, 5
 OPT_TILE_CFG_REINIT, OPT_CHUNK_REINIT = 6, 7
 
 _ERRNAMES = {1: "EINVAL", 2: "ENOMEM", 3: "EDEVICE", 4: "ETIMEOUT", 5: "ESTATE"}

@@ -317,6 +317,10 @@ int check_field(r3d_handle* h, int field) {
 // Airy velocity at the device clock (no-op unless r3d_set_velocity_airy);
 // maxima: also its CFL maxima into S.vmax.
 long long refresh_velocity(r3d_handle* h, bool maxima = false) {
+    if (h->launch_test) {
+        h->launch_test = 0;
+        launch_rejected(h->S.dt, h->stream);
+    }
     if (!h->airy) return 0;
     return launch_airy(h->L, h->field[R3D_U], h->field[R3D_W], fp32(h), h->coord, h->S.t, h->ap, h->sms,
                        maxima ? h->S.vmax : nullptr, h->stream);
@@ -391,6 +395,13 @@ int enqueue_step(r3d_handle* h) {
     h->launches += n;
     h->have_last_volume = true;
     return R3D_OK;
+}
+
+// Fails when a launch since the last check was rejected (a launch's own error,
+// also inside a capture, where the graph then lacks it).
+int check_launches(r3d_handle* h, const char* what) {
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? R3D_OK : cuda_fail(h, e, what);
 }
 
 // Reads and clears the device error flag raised by a bounded wait.
@@ -585,6 +596,7 @@ int r3d_ls_step(r3d_handle* h, double dt) {
         return fail(h, R3D_ESTATE, "no time step set (pass dt > 0, r3d_set_dt or r3d_cfl_dt first)");
     }
     h->launches += refresh_velocity(h);
+    if (int rc = check_launches(h, "velocity launch")) return rc;
     enqueue_step(h);
     h->wait_test = 0;  // a timeout-path test covers one step
     R3D_CUDA(h, cudaGetLastError());
@@ -596,20 +608,25 @@ int r3d_ls_step(r3d_handle* h, double dt) {
 // them by the velocity factor alone; the Airy generator rewrites u and w and
 // finds their maxima on the way, so only v's stays).  Taken per step they
 // were 41 of 1450 us at 256^3 and three of thirteen launches.
-void enqueue_run_start(r3d_handle* h, int adaptive) {
-    if (!adaptive) return;
+int enqueue_run_start(r3d_handle* h, int adaptive) {
+    if (!adaptive) return R3D_OK;
     h->launches += launch_vmax(h->L, h->field[R3D_U], h->field[R3D_V], h->field[R3D_W], fp32(h), h->S, h->stream);
     if (h->airy) {
         cudaMemsetAsync(h->S.vmax, 0, sizeof(unsigned long long), h->stream);
         cudaMemsetAsync(h->S.vmax + 2, 0, sizeof(unsigned long long), h->stream);
     }
+    return check_launches(h, "velocity maxima launch");
 }
 
 // The launches of one step of r3d_ls_run (the CFL step first when adaptive).
-void enqueue_run_step(r3d_handle* h, int adaptive) {
+// The stages follow only velocities and a time step that were launched: with
+// the maxima at 0 the step would be n47 1e10.
+int enqueue_run_step(r3d_handle* h, int adaptive) {
     h->launches += refresh_velocity(h, adaptive != 0);
     if (adaptive) h->launches += launch_dt(h->M.dxmin_cfl, h->desc.n47, h->S, h->airy, h->stream);
+    if (int rc = check_launches(h, "velocity and time step launches")) return rc;
     enqueue_step(h);
+    return check_launches(h, "step launches");
 }
 
 long long run_graph_key(const r3d_handle* h, int adaptive) {
@@ -635,10 +652,14 @@ int capture_step(r3d_handle* h, int adaptive) {
     cudaGraph_t g = nullptr;
     R3D_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     const long long before = h->launches;
-    enqueue_run_step(h, adaptive);
+    const int rc = enqueue_run_step(h, adaptive);
     h->graph_launches = h->launches - before;
     h->launches = before;
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
+    if (rc) {
+        if (e == cudaSuccess) cudaGraphDestroy(g);
+        return rc;
+    }
     if (e != cudaSuccess) return cuda_fail(h, e, "step graph capture");
     e = cudaGraphInstantiate(&h->step_graph, g, 0);
     cudaGraphDestroy(g);
@@ -658,14 +679,15 @@ int r3d_ls_run(r3d_handle* h, int nsteps, int adaptive) {
     const bool use_graph = nsteps >= 2 || (h->step_graph && h->graph_key == run_graph_key(h, adaptive));
     if (use_graph && !(h->step_graph && h->graph_key == run_graph_key(h, adaptive)))
         if (int rc = capture_step(h, adaptive)) return rc;
-    if (nsteps > 0) enqueue_run_start(h, adaptive);
+    if (nsteps > 0)
+        if (int rc = enqueue_run_start(h, adaptive)) return rc;
     for (int n = 0; n < nsteps; ++n) {
         if (use_graph) {
             R3D_CUDA(h, cudaGraphLaunch(h->step_graph, h->stream));
             h->launches += h->graph_launches;
             h->have_last_volume = true;
-        } else {
-            enqueue_run_step(h, adaptive);
+        } else if (int rc = enqueue_run_step(h, adaptive)) {
+            return rc;
         }
     }
     R3D_CUDA(h, cudaGetLastError());
@@ -1509,6 +1531,10 @@ int r3d_set_option(r3d_handle* h, int option, int value) {
             h->band64 = value ? 1 : 0;
             return R3D_OK;
         case R3D_OPT_WAIT_TEST: h->wait_test = value ? 1 : 0; return R3D_OK;
+        case R3D_OPT_LAUNCH_TEST:
+            h->launch_test = value ? 1 : 0;
+            if (value) drop_step_graph(h);
+            return R3D_OK;
         case R3D_OPT_TILE_CFG:
         case R3D_OPT_TILE_CFG_REINIT: {
             if (value < 0 || value >= tile_cfg_count()) return fail(h, R3D_EINVAL, "unknown tile configuration");
@@ -1541,6 +1567,7 @@ int r3d_get_option(r3d_handle* h, int option, int* value) {
         case R3D_OPT_CHUNK: *value = h->kc; return R3D_OK;
         case R3D_OPT_BAND64: *value = h->band64; return R3D_OK;
         case R3D_OPT_WAIT_TEST: *value = h->wait_test; return R3D_OK;
+        case R3D_OPT_LAUNCH_TEST: *value = h->launch_test; return R3D_OK;
         case R3D_OPT_TILE_CFG: *value = h->tile_cfg; return R3D_OK;
         case R3D_OPT_TILE_CFG_REINIT: *value = h->tile_cfg_r; return R3D_OK;
         case R3D_OPT_CHUNK_REINIT: *value = h->kc_r; return R3D_OK;

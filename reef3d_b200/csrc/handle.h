@@ -68,6 +68,7 @@ struct r3d_handle {
     int tile_cfg_r = 0;
     int band64 = 1;
     int wait_test = 0;  // R3D_OPT_WAIT_TEST: armed for the next r3d_ls_step
+    int launch_test = 0;  // R3D_OPT_LAUNCH_TEST: armed for the next step's first launch
     CUtensorMap map[3];    // stage inputs phi, WORK1, WORK2 for tile_cfg
     CUtensorMap map_r[3];  // the same for tile_cfg_r
     // set while the instance is a member of a batch: calls on the handle

@@ -319,6 +319,8 @@ struct TileArgs;
 size_t tile_smem_bytes(int cfg);
 dim3 tile_grid(const Layout& L, int kc, int cfg);
 int launch_set_scalar(double* dst, double value, cudaStream_t st);
+// A launch the runtime refuses (2048 threads in a block): nothing runs.
+void launch_rejected(double* dst, cudaStream_t st);
 int launch_init_fields(const Layout& L, const double* xc, const double* xf, int ns, const double* sph, int nm,
                        const double* modes, bool fp32, void* phi, void* u, void* v, void* w, cudaStream_t st);
 

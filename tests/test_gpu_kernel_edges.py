@@ -231,3 +231,35 @@ def test_airy_instances_leave_each_other_their_shared_memory():
     finally:
         long.close()
         short.close()
+
+
+@pytest.mark.parametrize("call", ["step", "run1", "run3"])
+@pytest.mark.parametrize("airy", [False, True])
+def test_rejected_launch_leaves_the_level_set(call, airy):
+    """A step whose first launch the runtime refuses fails before a stage runs
+    and leaves no graph behind that lacks the launch: the next run is a fresh
+    instance's."""
+    def make():
+        ls = instance((40, 24, 18))
+        ls.init_spheres_tg([(0.5, 0.5, 0.5, 0.25)], [(1, 0.5), (2, 0.3)])
+        if airy:
+            ls.set_time(0.0)
+            ls.set_velocity_airy(0.05, 2.0, 0.5)
+        return ls
+    a, b = make(), make()
+    try:
+        before = dense(a)
+        dt = a.cfl_dt()
+        a.set_option(r3d.OPT_LAUNCH_TEST, 1)
+        with pytest.raises(r3d.R3DError):
+            a.step(dt) if call == "step" else a.run(int(call[3:]), adaptive=True)
+        a.sync()
+        assert a.get_option(r3d.OPT_LAUNCH_TEST) == 0
+        assert np.array_equal(dense(a), before) and a.time() == 0.0
+        for ls in (a, b):
+            ls.run(3, adaptive=True)
+            ls.sync()
+        assert a.time() == b.time() and np.array_equal(dense(a), dense(b))
+    finally:
+        a.close()
+        b.close()
