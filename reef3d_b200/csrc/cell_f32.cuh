@@ -1,6 +1,6 @@
 // FP32 cell operators shared by the per-instance kernels (kernels_f32.cu)
 // and the batched persistent kernels (kernels_batch.cu): one cell per call,
-// stencils read through the read-only cache.
+// fields read by plain loads (launch_step), tables through the read-only cache.
 #pragma once
 
 #include "stencil_f32.cuh"
@@ -8,8 +8,6 @@
 namespace r3d {
 namespace f32c {
 
-// plain loads: the stage that writes f may still drain when the kernel is
-// launched (launch_step)
 __device__ __forceinline__ void load7(const float* f, long long c, long long s, float* o) {
 #pragma unroll
     for (int m = 0; m < 7; ++m) o[m] = f[c + (m - 3) * s];
@@ -106,19 +104,18 @@ __device__ __forceinline__ float deriv_tables_df(const float* fv, const double* 
     return f32::weno5_tables(wt + 18 * (2 * t + off), plus, q[0], q[1], q[2], q[3], q[4]);
 }
 
-__device__ __forceinline__ void load7d(const double* __restrict__ f, long long c, long long s, double* o) {
+__device__ __forceinline__ void load7d(const double* __restrict__ body, long long c, long long s, double* o) {
 #pragma unroll
-    for (int m = 0; m < 7; ++m) o[m] = __ldg(f + c + (m - 3) * s);
+    for (int m = 0; m < 7; ++m) o[m] = __ldg(body + c + (m - 3) * s);
 }
 
 // DF: the direct-forcing stencils of g.x45 over g.body (table form).
 template <bool TWO_D, bool UNIFORM, bool DF = false>
-__device__ __forceinline__ float conv_L(const KGrid<float>& g, const float* f,
-                                        const float* __restrict__ u, const float* __restrict__ v,
-                                        const float* __restrict__ w, long long c, int i, int j, int k, float vs) {
+__device__ __forceinline__ float conv_L(const KGrid<float>& g, const float* f, const float* u, const float* v,
+                                        const float* w, long long c, int i, int j, int k, float vs) {
     const long long sy = g.L.sy, sz = g.L.sz;
-    const float ia = 0.5f * vs * (__ldg(u + c) + __ldg(u + c - 1));
-    const float ka = 0.5f * vs * (__ldg(w + c) + __ldg(w + c - sz));
+    const float ia = 0.5f * vs * (u[c] + u[c - 1]);
+    const float ka = 0.5f * vs * (w[c] + w[c - sz]);
     float fv[7];
     double hv[7];
     auto axis = [&](long long s, int a, int t, bool plus) {
@@ -136,7 +133,7 @@ __device__ __forceinline__ float conv_L(const KGrid<float>& g, const float* f,
         l -= ia * axis(1, 0, i + 5, ia < 0.0f);
     }
     if (!TWO_D) {
-        const float ja = 0.5f * vs * (__ldg(v + c) + __ldg(v + c - sy));
+        const float ja = 0.5f * vs * (v[c] + v[c - sy]);
         if (ja != 0.0f) {
             load7(f, c, sy, fv);
             l -= ja * axis(sy, 1, j + 5, ja < 0.0f);

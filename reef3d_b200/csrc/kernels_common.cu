@@ -204,7 +204,7 @@ __global__ void dt_kernel(unsigned long long* vm, const double* vscale, double d
 
 // --------------------------------------------------------------- volume
 // Second pass: one block sums the per-block partials in a fixed order.
-__global__ void volume_reduce_kernel(const double* __restrict__ partial, long long n, double* out, double* t,
+__global__ void volume_reduce_kernel(const double* partial, long long n, double* out, double* t,
                                      double* vscale, const double* dt, double period) {
     step_next();
     step_wait();
@@ -368,9 +368,9 @@ __global__ void __launch_bounds__(256) airy_kernel(Layout L, T* __restrict__ u, 
 // src/gc_neumann.cpp:29-54; 2D skips y), and the volume partials of
 // volume_direct_kernel.
 template <typename T, bool STEP>
-__global__ void fluid_kernel(Layout L, const T* __restrict__ phi, T* __restrict__ ro, T* __restrict__ visc,
-                             const double* __restrict__ dxn, const double* __restrict__ dyn,
-                             const double* __restrict__ dzn, double psi, FluidConst fc, double* partial) {
+__global__ void fluid_kernel(Layout L, const T* phi, T* ro, T* visc, const double* __restrict__ dxn,
+                             const double* __restrict__ dyn, const double* __restrict__ dzn, double psi, FluidConst fc,
+                             double* partial) {
     if (STEP) {
         step_next();
         step_wait();
@@ -544,8 +544,8 @@ constexpr int kIoThreads = 1024;
 // so the FP64 sum rounds exactly as the reference's loop does.  zval is
 // valid in thread 0, count in every thread.
 template <typename T>
-__device__ __forceinline__ bool crossing_height(const Layout& L, const T* __restrict__ phi, int i, const IoParams& p,
-                                                int j, int k, double& h) {
+__device__ __forceinline__ bool crossing_height(const Layout& L, const T* phi, int i, const IoParams& p, int j, int k,
+                                                double& h) {
     const long long c = (long long)(k + L.gz) * L.sz + (long long)(j + L.gy) * L.sy + (i + L.gx);
     const double a = static_cast<double>(phi[c]), b = static_cast<double>(phi[c + L.sz]);
     if (!(a >= 0.0 && b < 0.0)) return false;
@@ -655,7 +655,7 @@ __device__ void io_levels(const In& in, const Out& out, const IoParams& p) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kIoThreads) io_level_kernel(Layout L, const T* __restrict__ phi, IoParams p) {
+__global__ void __launch_bounds__(kIoThreads) io_level_kernel(Layout L, const T* phi, IoParams p) {
     step_next();
     step_wait();
     io_levels(CellHeights<T>{L, phi, p, -1}, CellHeights<T>{L, phi, p, L.nx - 1}, p);
@@ -690,8 +690,7 @@ __global__ void __launch_bounds__(kIoThreads) io_fold_kernel(const double* __res
 // phi's, outflow ghosts copy phi's or hold F62 - ZP (F62 set, B77 = 2).
 // One thread per (j,k) of the x faces.
 template <typename T>
-__global__ void __launch_bounds__(256) io_ghost_kernel(Layout L, T* __restrict__ phi, T* __restrict__ a1,
-                                                       T* __restrict__ a2, IoParams p, int step) {
+__global__ void __launch_bounds__(256) io_ghost_kernel(Layout L, T* phi, T* a1, T* a2, IoParams p, int step) {
     step_next();
     step_wait();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;

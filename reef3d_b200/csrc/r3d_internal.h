@@ -130,8 +130,11 @@ struct Scratch {
 // (programmatic dependent launch): the launch, 1 to 2 us, is a third of a
 // small grid's stage.  A kernel launched this way calls step_wait() before it
 // touches anything another kernel writes; the wait returns when every
-// earlier kernel is done and its writes are visible.  step_next() allows the
-// successor to be launched.  For grids of one wave (the successor finds room
+// earlier kernel is done and its writes are visible.  Whatever another kernel of
+// the step writes (fields, velocities, partials, scalars) is read by plain loads
+// through pointers without __restrict__: __ldg or a restricted parameter says
+// that it stays unwritten for the kernel's whole life, and lets the load move
+// above the wait.  step_next() allows the successor to be launched.  For grids of one wave (the successor finds room
 // beside them): a 2D flume of 600 x 75 cells stepped one call at a time
 // 1.64 -> 1.37 ms for ten steps, 128 x 128 in a graph 3.08 -> 2.92 ms for 60;
 // with several waves the wait of every block costs more than it hides (256^3

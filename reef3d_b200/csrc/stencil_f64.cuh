@@ -12,9 +12,9 @@
 namespace r3d {
 namespace f64 {
 
-// The level set f is read by plain loads, not through the read-only path: a
-// stage may be launched while the one that writes f still drains
-// (launch_step), so f does not stay unwritten for the kernel's whole life.
+// The fields (level set, face velocities) are read by plain loads through
+// pointers without __restrict__ (launch_step); the tables, which nothing writes
+// after creation, go through the read-only path.
 
 // a / b rounded to nearest from r = 1/b rounded to nearest (the IEEE
 // reciprocal, tabulated per grid spacing): q0 = a r, then two residual
@@ -211,13 +211,11 @@ __device__ __forceinline__ double deriv_df(const double* f, const double* __rest
 // The stored face velocities are multiplied by vs (1 leaves them exact).
 // DF: the direct-forcing stencils of g.x45 (g.body) replace the plain ones.
 template <bool TWO_D, bool DF = false>
-__device__ __forceinline__ double conv_L(const KGrid<double>& g, const double* f,
-                                         const double* __restrict__ u, const double* __restrict__ v,
-                                         const double* __restrict__ w, long long c, int i, int j, int k,
-                                         double vs) {
+__device__ __forceinline__ double conv_L(const KGrid<double>& g, const double* f, const double* u, const double* v,
+                                         const double* w, long long c, int i, int j, int k, double vs) {
     const long long sy = g.L.sy, sz = g.L.sz;
-    const double iadvec = 0.5 * (vs * __ldg(u + c) + vs * __ldg(u + c - 1));
-    const double kadvec = 0.5 * (vs * __ldg(w + c) + vs * __ldg(w + c - sz));
+    const double iadvec = 0.5 * (vs * u[c] + vs * u[c - 1]);
+    const double kadvec = 0.5 * (vs * w[c] + vs * w[c - sz]);
     auto axis = [&](long long s, int a, int t, bool plus) {
         if (DF) return deriv_df(f, g.body, c, s, g.dxp[a], g.wt[a], t, plus, g.x45, g.df_thr);
         return deriv(f, c, s, g.dpr[a], g.wt[a], t, plus);
@@ -227,7 +225,7 @@ __device__ __forceinline__ double conv_L(const KGrid<double>& g, const double* f
     if (iadvec == 0.0) grad = 0.0;
     double l = -iadvec * grad;
     if (!TWO_D) {
-        const double jadvec = 0.5 * (vs * __ldg(v + c) + vs * __ldg(v + c - sy));
+        const double jadvec = 0.5 * (vs * v[c] + vs * v[c - sy]);
         grad = axis(sy, 1, j + 5, jadvec < 0.0);
         if (jadvec == 0.0) grad = 0.0;
         l -= jadvec * grad;
