@@ -37,7 +37,7 @@ UNITS = [
     ("serve.cpp", []),
     ("state.cpp", []),
 ]
-HEADERS = ["r3d_internal.h", "stencil_f64.cuh", "stencil_f32.cuh", "tile_host.h", "cell_f32.cuh", "handle.h", "batch_internal.h"]
+HEADERS = ["r3d_internal.h", "quotient.h", "stencil_f64.cuh", "stencil_f32.cuh", "tile_host.h", "cell_f32.cuh", "handle.h", "batch_internal.h"]
 
 
 def nvcc():

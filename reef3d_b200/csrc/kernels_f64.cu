@@ -12,9 +12,9 @@ namespace {
 constexpr int kBX = 32, kBY = 4;
 // Resident blocks per SM the stage kernels are register-limited for: 64
 // registers in the convection; 80 in the reinitialisation, which holds the six
-// face differences of an axis through the weights and spills in 64 (256^3,
-// us per stage 1 / 2: 776 / 744 at eight blocks against 816 / 847 at six;
-// 813 / 854 at six against 926 / 954 at eight).
+// face differences of an axis through the weights and spills in 64 (926 / 954
+// us per stage 1 / 2 at 256^3 against 813 / 854, with the weights' quotients of
+// that time).
 constexpr int kConvBlocks = 8, kReiniBlocks = 6;
 
 struct StageArgs {

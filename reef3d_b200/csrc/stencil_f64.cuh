@@ -6,6 +6,7 @@
 // spacings through div_rn, which forms the same quotient).
 #pragma once
 
+#include "quotient.h"
 #include "r3d_internal.h"
 
 
@@ -32,38 +33,16 @@ __device__ __forceinline__ double div_rn(double a, double b, double r) {
     return fma(fma(-b, q1, a), r, q1);
 }
 
-// 1/b to within an ulp for a normal b: the hardware's approximation (relative
-// error e below 2^-23) and one cubic Newton step y (1 + e + e^2), whose error
-// is e^3.
-__device__ __forceinline__ double rcp_f64(double b) {
+// A bound of 1/b (reciprocal_below) from the hardware's approximation, which
+// takes and gives the upper 32 bits of a double: |1 - b y| < 2^-19.93, the
+// largest over all 2^20 mantissas with the low word all zeros and all ones.
+__device__ __forceinline__ double rcp_below(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double e = fma(-b, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-
-// a / b from y, an approximation of 1/b to a few ulps: the quotient a y
-// corrected once by its residual, which a fused multiply-add gives exactly
-// (Markstein, as in div_rn).  Before its last rounding the result is within
-// 2^-102 of a/b relative to it, so it is the IEEE quotient unless a/b lies
-// that close to the middle of two doubles (one in 2^49 random quotients).
-__device__ __forceinline__ double div_y(double a, double b, double y) {
-    const double q = a * y;
-    return fma(fma(-b, q, a), y, q);
+    return reciprocal_below(b, y);
 }
 
 __device__ __forceinline__ double2 ldg2(const double* p) { return __ldg(reinterpret_cast<const double2*>(p)); }
-
-// The nonlinear weights c_r / (s_r^2 sum), sum = c0/s0^2 + c1/s1^2 + c2/s2^2,
-// by the compiler's divisions: any A = s0^2, B = s1^2, C = s2^2 (overflowed,
-// infinite, NaN).
-__device__ __noinline__ void weights_any(double c0, double c1, double c2, double A, double B, double C, double* w) {
-    const double eps = 0.0;
-    const double sum = c0 / A + c1 / B + c2 / C;
-    w[0] = c0 / (eps + A * sum);
-    w[1] = c1 / (eps + B * sum);
-    w[2] = c2 / (eps + C * sum);
-}
 
 // WENO5 derivative from the divided differences q1..q5 of the upwind set,
 // node tables of index t and the side: the record W = wt + 18 (2t + side)
@@ -71,15 +50,10 @@ __device__ __noinline__ void weights_any(double c0, double c1, double c2, double
 // Minus side: IS src/weno_nug_func.h:48-60, weights :133-143,
 // reconstruction src/weno_hj_df_nug.cpp:155-159.  Plus side: :61-73,
 // :144-153, :186-190.  epsilon = 0, psi = 1e-6 (src/weno_nug_func.cpp:26).
-//
-// The six quotients of the weights have 1/A, 1/B, 1/C and 1/sum in common
-// (1/(A sum) = 1/A 1/sum to a few ulps): four reciprocals and 33 FP64
-// operations without range checks, where six IEEE divisions took about 50
-// and 60 others.  Where one of A, B, C (1e-12 and up by psi) leaves
-// [2^-511, 2^499), compared on the high words, weights_any forms them.
-__device__ __forceinline__ double weno5(const double* __restrict__ W, bool plus, double q1, double q2, double q3,
-                                        double q4, double q5) {
-    const double2 w01 = ldg2(W + 0), w23 = ldg2(W + 2), w45 = ldg2(W + 4), w67 = ldg2(W + 6);
+
+// The squared indicators (IS + psi)^2 of the three stencils.
+__device__ __forceinline__ void squares(const double* __restrict__ W, double q1, double q2, double q3, double q4,
+                                        double q5, double& A, double& B, double& C) {
     const double2 w89 = ldg2(W + 8), wab = ldg2(W + 10), wcd = ldg2(W + 12), wef = ldg2(W + 14);
     const double2 wgh = ldg2(W + 16);
     const double S[9] = {w89.y, wab.x, wab.y, wcd.x, wcd.y, wef.x, wef.y, wgh.x, wgh.y};
@@ -90,33 +64,21 @@ __device__ __forceinline__ double weno5(const double* __restrict__ W, bool plus,
     const double is2 = S[3] * dq23 * dq23 + S[4] * (dq43) * (dq23) + S[5] * dq43 * dq43;
     const double is3 = S[6] * dq12 * dq12 + S[7] * (dq32) * (dq12) + S[8] * dq32 * dq32;
     const double a = is1 + psi, b = is2 + psi, c = is3 + psi;
-    const double c0 = w67.x, c1 = w67.y, c2 = w89.x;
-    const double A = a * a, B = b * b, C = c * c;
-    double w1, w2, w3;
-    const unsigned lo = 0x20000000u;  // high word of 2^-511
-    const unsigned top = max(max((unsigned)__double2hiint(A) - lo, (unsigned)__double2hiint(B) - lo),
-                             (unsigned)__double2hiint(C) - lo);
-    if (top < 0x5f200000u - lo) {  // all from 2^-511 to below 2^499
-        const double yA = rcp_f64(A), yB = rcp_f64(B), yC = rcp_f64(C);
-        const double sum = div_y(c0, A, yA) + div_y(c1, B, yB) + div_y(c2, C, yC);
-        const double ys = rcp_f64(sum);
-        w1 = div_y(c0, A * sum, yA * ys);
-        w2 = div_y(c1, B * sum, yB * ys);
-        w3 = div_y(c2, C * sum, yC * ys);
-    } else {
-        double w[3];
-        weights_any(c0, c1, c2, A, B, C, w);
-        w1 = w[0];
-        w2 = w[1];
-        w3 = w[2];
-    }
+    A = a * a;
+    B = b * b;
+    C = c * c;
+}
+
+// The weighted reconstruction.  The two sides' differ only in which
+// differences enter and in two signs (minus side :155-159, plus side
+// :186-190); selecting those operands keeps every rounding of either side:
+//   w1 (q4 + Q0 (q3-q4) -+ Q1 (q5-q4))
+//   w2 (q3 + Q2 x2 - Q3 y2)   x2, y2 = (q4-q3), (q2-q3)  [plus: swapped]
+//   w3 (q2 + Q4 x3 +- Q5 y3)  x3, y3 = (q1-q2), (q3-q2)  [plus: swapped]
+__device__ __forceinline__ double reconstruct(const double* __restrict__ W, bool plus, double q1, double q2,
+                                              double q3, double q4, double q5, double w1, double w2, double w3) {
+    const double2 w01 = ldg2(W + 0), w23 = ldg2(W + 2), w45 = ldg2(W + 4);
     const double Q0 = w01.x, Q1 = w01.y, Q2 = w23.x, Q3 = w23.y, Q4 = w45.x, Q5 = w45.y;
-    // The two sides' reconstructions differ only in which differences enter
-    // and in two signs (minus side :155-159, plus side :186-190); selecting
-    // those operands keeps every rounding of either side:
-    //   w1 (q4 + Q0 (q3-q4) -+ Q1 (q5-q4))
-    //   w2 (q3 + Q2 x2 - Q3 y2)   x2, y2 = (q4-q3), (q2-q3)  [plus: swapped]
-    //   w3 (q2 + Q4 x3 +- Q5 y3)  x3, y3 = (q1-q2), (q3-q2)  [plus: swapped]
     const double t1 = Q1 * (q5 - q4);
     const double x2 = plus ? (q2 - q3) : (q4 - q3), y2 = plus ? (q4 - q3) : (q2 - q3);
     const double x3 = plus ? (q3 - q2) : (q1 - q2), y3 = plus ? (q1 - q2) : (q3 - q2);
@@ -124,6 +86,49 @@ __device__ __forceinline__ double weno5(const double* __restrict__ W, bool plus,
     return w1 * (q4 + Q0 * (q3 - q4) + (plus ? t1 : -t1))
          + w2 * (q3 + Q2 * x2 - Q3 * y2)
          + w3 * (q2 + Q4 * x3 + (plus ? -t3 : t3));
+}
+
+// The evaluation with the compiler's divisions: any indicators (overflowed,
+// infinite, NaN).
+__device__ __noinline__ double weno5_any(const double* __restrict__ W, bool plus, double q1, double q2, double q3,
+                                         double q4, double q5) {
+    double A, B, C;
+    squares(W, q1, q2, q3, q4, q5, A, B, C);
+    const double c0 = __ldg(W + 6), c1 = __ldg(W + 7), c2 = __ldg(W + 8);
+    const double eps = 0.0;
+    const double sum = c0 / A + c1 / B + c2 / C;
+    return reconstruct(W, plus, q1, q2, q3, q4, q5, c0 / (eps + A * sum), c1 / (eps + B * sum), c2 / (eps + C * sum));
+}
+
+// The six quotients of the weights have 1/A, 1/B, 1/C and 1/sum in common
+// (1/(A sum) from 1/A and 1/sum): four reciprocals, and each quotient from both
+// ends of its bracket (bracket_div), 46 FP64 operations and a few others.
+// Where the ends round apart, about one evaluation in 2^17, or one of A, B, C
+// (1e-12 and up by psi) leaves [2^-511, 2^499), compared on the high words,
+// weno5_any divides: all are the IEEE quotients.  At 256^3, us per stage 1 / 2:
+// convection 798 / 830 with six IEEE divisions, 709 / 741 so; reinitialisation
+// 838 / 882 and 791 / 840.  (One residual correction per quotient with the
+// product of two reciprocals, without the second end, took 778 / 747 and 813 /
+// 855, with more spilled registers, and was an ulp off where a quotient lies next
+// to the middle of two doubles.)
+__device__ __forceinline__ double weno5(const double* __restrict__ W, bool plus, double q1, double q2, double q3,
+                                        double q4, double q5) {
+    double A, B, C;
+    squares(W, q1, q2, q3, q4, q5, A, B, C);
+    const double2 w67 = ldg2(W + 6);
+    const double c0 = w67.x, c1 = w67.y, c2 = __ldg(W + 8);
+    const unsigned lo = 0x20000000u, hi = 0x5f200000u;  // high words of 2^-511, 2^499
+    const unsigned top = max(max((unsigned)__double2hiint(A) - lo, (unsigned)__double2hiint(B) - lo),
+                             (unsigned)__double2hiint(C) - lo);
+    uint32_t apart = top < hi - lo ? 0 : 1;
+    const double yA = rcp_below(A), yB = rcp_below(B), yC = rcp_below(C);
+    const double sum = bracket_div(c0, A, yA, apart) + bracket_div(c1, B, yB, apart) + bracket_div(c2, C, yC, apart);
+    const double ys = rcp_below(sum);
+    const double w1 = bracket_div(c0, A * sum, yA * ys, apart);
+    const double w2 = bracket_div(c1, B * sum, yB * ys, apart);
+    const double w3 = bracket_div(c2, C * sum, yC * ys, apart);
+    if (apart) return weno5_any(W, plus, q1, q2, q3, q4, q5);
+    return reconstruct(W, plus, q1, q2, q3, q4, q5, w1, w2, w3);
 }
 
 // Upwind-biased derivative along one axis (stride s) at linear index c,
