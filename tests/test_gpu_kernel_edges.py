@@ -80,6 +80,45 @@ def test_steep_fields_fp32(scale, tiled):
     assert relmax(res[1], res[0]) <= 1e-3 * n * 64 * EPS32 + 4 * EPS32
 
 
+@pytest.mark.parametrize("dims,stretch,tiled,roundings", [
+    ((128, 1, 128), 0.0, 1, 9), ((301, 1, 157), 0.0, 1, 9), ((97, 61, 120), 0.0, 0, 9), ((50, 111, 83), 0.0, 1, 9),
+    ((413, 1, 211), 0.3, 1, 13), ((96, 80, 112), 0.3, 1, 13)])
+def test_convection_error_fp32(dims, stretch, tiled, roundings):
+    """The FP32 convection operator against FP64's on the same (FP32) values, by
+    its 2-norm: the roundings on the way of a value's leading part (difference,
+    two of the reconstruction, the correction's sum, 1/h, three of the
+    velocity and its product, the axes' sum: 9; quotient, its reciprocal's and
+    two of the tables: 13), each 0.42 2^-24 rms for mantissas spread over a
+    binade, added in quadrature.  Weights add nothing of that order: they
+    multiply differences of reconstructions."""
+    rng = np.random.default_rng(dims[0])
+    nodes = []
+    for n in dims:
+        length = 1.0 if n > 1 else 1.0 / dims[0]
+        x = r3d.uniform_nodes(n, length)
+        nodes.append(x + (stretch * np.sin(2 * np.pi * x / length) * length / (2 * np.pi) if n > 1 else 0.0))
+    spheres = [(*map(float, rng.uniform(0.2, 0.8, 3)), float(rng.uniform(0.05, 0.2))) for _ in range(4)]
+    modes = [(int(rng.integers(1, 4)), float(rng.normal(0.0, 0.5))) for _ in range(4)]
+    with instance(dims, r3d.FP64, nodes) as ls:
+        ls.init_spheres_tg(spheres, modes)
+        ls.run(10)
+        fields = {f: ls.download(f).astype(np.float32).astype(np.float64) for f in (r3d.PHI, r3d.U, r3d.V, r3d.W)}
+    out = []
+    for prec in (r3d.FP64, r3d.FP32):
+        with instance(dims, prec, nodes) as ls:
+            if prec == r3d.FP32:
+                ls.set_option(r3d.OPT_TILED, tiled)
+            for f, a in fields.items():
+                ls.upload(f, a)
+            ls.ghost_fill()
+            ls.set_dt(1e4)  # phi + dt L is dt L
+            ls.stage(r3d.STAGE_CONVECTION, 1)
+            ls.sync()
+            out.append(ls.download(r3d.WORK1, r3d.LAYOUT_DENSE))
+    err = np.linalg.norm(out[1] - out[0]) / np.linalg.norm(out[0])
+    assert err <= 0.42 * EPS32 * np.sqrt(roundings)
+
+
 @pytest.mark.parametrize("scale", [1.0, 1e20, 1e34, 1e35, 1e36, 1e70, 1e80])
 def test_fp64_weights_range(port_lib, scale):
     """The FP64 operators bit for bit where the squared indicators pass 2^499
