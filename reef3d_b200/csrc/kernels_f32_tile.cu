@@ -180,8 +180,13 @@ __device__ __noinline__ double band_axis(float f0, float f1, float f2_, float f3
 __device__ __forceinline__ float band_rhs(float f0f, double g2, float deltax) {
     const double f0 = f0f, dl = deltax;
     const double dn = sqrt(g2);
-    double S = f0 * rsqrt(f0 * f0 + g2 * dl * dl);
-    if (S != S) S = 1.0;
+    const double x = f0 * f0 + g2 * dl * dl;
+    // f0 / sqrt(x): one Newton step on the reciprocal root (an ulp off) costs
+    // nothing here and leaves no more rounding than a root and a division,
+    // which took 143 instead of 140 us of a 256^3 stage
+    const double y = rsqrt(x), S0 = f0 * y;
+    double S = fma(0.5 * S0, fma(-(x * y), y, 1.0), S0);
+    if (S0 != S0) S = 1.0;
     return (float)(S - S * dn);
 }
 
