@@ -107,9 +107,14 @@ __device__ __forceinline__ float2 sel2(bool cx, bool cy, float2 a, float2 b) {
 // Ratios need no scaling against the FP32 range whatever h is.  One of p, q
 // is always above 0.05 (s1 >= 0.24 c^2, s3 >= 0.24 b^2, s2 <= 2 (b^2 + c^2)
 // plus the psi terms), so the denominator cannot vanish; 1e-15 (s1 + s3)
-// added to s2 bounds the ratios by 1e15, so that no square of a field far
-// from a distance function leaves the FP32 range (the weight it changes is
-// below 1e-12).
+// added to s2 bounds the ratios by 1e15, so that P and Q stay in range.  A
+// denominator that leaves it (P Q above 2.7e37) gives F, off by weights below
+// 1e-8.  The range ends where a second difference squared does, at 1e19 (1e16
+// and up in the reinitialisation, which squares gradients too): not finite
+// there.  The error is 2^-24 of the largest second difference in the stencil,
+// spikes of any size included; the form with three products of squared
+// indicators, clamped at 1e6, was off by half a spike's size from 10 up and not
+// finite from 1e16 on.
 // 31 packed operations and no clamps after the selects, where the form with
 // three products of squared indicators took 37 and 6, and half the distinct
 // constants (the registers that hold them limit the CTAs per SM).  With the

@@ -80,6 +80,42 @@ def test_steep_fields_fp32(scale, tiled):
     assert relmax(res[1], res[0]) <= 1e-3 * n * 64 * EPS32 + 4 * EPS32
 
 
+@pytest.mark.parametrize("spike", [10.0, 1e3, 1e6, 1e9, 1e12, 1e16])
+@pytest.mark.parametrize("kind", [r3d.STAGE_CONVECTION, r3d.STAGE_REINIT])
+@pytest.mark.parametrize("f49", [1, 0])
+def test_spikes_fp32(spike, kind, f49):
+    """Isolated values far above the rest, up to the ends of the packed form's
+    range: finite, and FP64's to the rounding of the largest value within three
+    cells."""
+    from scipy.ndimage import maximum_filter
+    if kind == r3d.STAGE_REINIT and spike > 1e12:
+        pytest.skip("gradients beyond the squares' range")
+    n = 40
+    rng = np.random.default_rng(7)
+    x = (np.arange(n) + 0.5) / n
+    phi = (x[:, None, None] - 0.45) + 0.2 * np.sin(5 * x)[None, :, None] * np.cos(4 * x)[None, None, :]
+    at = rng.integers(0, n, (40, 3))
+    at[:4] = [[0, 0, 0], [n - 1, n - 1, n - 1], [20, 0, n - 1], [n - 1, 7, 0]]
+    for k, j, i in at:
+        phi[k, j, i] = spike * rng.uniform(-1.0, 1.0)
+    phi = phi.astype(np.float32).astype(np.float64)
+    out = []
+    for prec in (r3d.FP64, r3d.FP32):
+        with instance((n, n, n), prec, f49=f49) as ls:
+            ls.init_spheres_tg([(0.5, 0.5, 0.5, 0.2)], [(1, 0.5), (2, 0.25)])
+            ls.upload(r3d.PHI, phi, r3d.LAYOUT_DENSE)
+            ls.ghost_fill()
+            ls.set_dt(1.0 / n)
+            ls.stage(kind, 1)
+            ls.sync()
+            out.append(ls.download(r3d.WORK1, r3d.LAYOUT_DENSE))
+    assert np.all(np.isfinite(out[1]))
+    # a derivative times h is at most 4 differences of values within three cells,
+    # three axes of them times a velocity (pseudo-step) of at most h a step
+    size = maximum_filter(np.abs(phi), size=7, mode="nearest")
+    assert np.all(np.abs(out[1] - out[0]) <= 16 * EPS32 * (size + 1.0))
+
+
 @pytest.mark.parametrize("dims,stretch,tiled,roundings", [
     ((128, 1, 128), 0.0, 1, 9), ((301, 1, 157), 0.0, 1, 9), ((97, 61, 120), 0.0, 0, 9), ((50, 111, 83), 0.0, 1, 9),
     ((413, 1, 211), 0.3, 1, 13), ((96, 80, 112), 0.3, 1, 13)])
