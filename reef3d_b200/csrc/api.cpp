@@ -121,9 +121,13 @@ void fill_kgrid(r3d_handle* h, KGrid<T>& g, T* base, std::vector<T>& host) {
     g.f43 = h->desc.f43;
     g.f49 = h->desc.f49;
     g.psi = h->M.psi;
+    // undivided differences square h: outside these spacings 1e-6 h^2 or a squared
+    // difference leaves the FP32 range, and a uniform grid takes the tables
+    bool undivided = h->M.uniform;
+    for (int a = 0; a < 3; ++a) undivided = undivided && h->M.h[a] > 1.0e-15 && h->M.h[a] < 1.0e16;
     for (int a = 0; a < 3; ++a) {
-        g.h[a] = h->M.uniform ? (float)h->M.h[a] : 0.0f;
-        g.rh[a] = h->M.uniform ? (float)(1.0 / h->M.h[a]) : 0.0f;
+        g.h[a] = undivided ? (float)h->M.h[a] : 0.0f;
+        g.rh[a] = undivided ? (float)(1.0 / h->M.h[a]) : 0.0f;
     }
     g.eps_u = 1.0e-6f;
 }

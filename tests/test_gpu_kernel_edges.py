@@ -116,6 +116,33 @@ def test_spikes_fp32(spike, kind, f49):
     assert np.all(np.abs(out[1] - out[0]) <= 16 * EPS32 * (size + 1.0))
 
 
+@pytest.mark.parametrize("dims", [(32, 32, 32), (32, 1, 32)])
+@pytest.mark.parametrize("e", [-56, -50, -44, -40, -30, 0, 40, 46, 52, 56, 60, 64])
+def test_spacings_fp32(e, dims):
+    """Boxes of 2^e a side, flat parts included: the kernels square h, and leave
+    the tiles, then the undivided differences, where that leaves the FP32
+    range.  Scaling by a power of two changes nothing else: FP64's convection
+    to eight roundings of the values."""
+    s = 2.0 ** e
+    x = (np.arange(32) + 0.5) / 32
+    phi = np.sin(5 * x)[None, None, :] * np.cos(4 * x[:dims[1]])[None, :, None] + 0.5 * np.sin(6 * x)[:, None, None]
+    phi[:, :, :8] = 0.25
+    phi = phi.astype(np.float32).astype(np.float64)
+    nodes = [r3d.uniform_nodes(n, s if n > 1 else s / 32) for n in dims]
+    out = []
+    for prec in (r3d.FP64, r3d.FP32):
+        with instance(dims, prec, nodes) as ls:
+            for f in (r3d.U, r3d.V, r3d.W):
+                ls.upload(f, np.full(ls.reef3d_shape, 0.5))
+            ls.upload(r3d.PHI, phi * s, r3d.LAYOUT_DENSE)
+            ls.ghost_fill()
+            ls.set_dt(s / 64)
+            ls.stage(r3d.STAGE_CONVECTION, 1)
+            ls.sync()
+            out.append(ls.download(r3d.WORK1, r3d.LAYOUT_DENSE) / s)
+    assert np.max(np.abs(out[1] - out[0])) <= 8 * EPS32
+
+
 @pytest.mark.parametrize("dims,stretch,tiled,roundings", [
     ((128, 1, 128), 0.0, 1, 9), ((301, 1, 157), 0.0, 1, 9), ((97, 61, 120), 0.0, 0, 9), ((50, 111, 83), 0.0, 1, 9),
     ((413, 1, 211), 0.3, 1, 13), ((96, 80, 112), 0.3, 1, 13)])
