@@ -347,14 +347,17 @@ void save_cache(const char* path) {
     }
 }
 
-// The z chunks and the (tile configuration, z chunk) candidates of the
-// autotuners.
+// The z chunks the autotuners try, and the (tile configuration, z chunk)
+// candidates around a starting chunk: from above half of it to four times it,
+// at most seven of them.  A 256^3 sweep launches every candidate 24 times, so
+// chunks that suit grids a tenth its size cost it a fifth of the sweep.
 constexpr int kChunks[] = {2, 4, 6, 7, 8, 10, 12, 16, 32};
 
-std::vector<std::pair<int, int>> tile_candidates() {
+std::vector<std::pair<int, int>> tile_candidates(int start) {
     std::vector<std::pair<int, int>> out;
     for (int c = 0; c < tile_cfg_count(); ++c)
-        for (int kc : kChunks) out.push_back({c, kc});
+        for (int kc : kChunks)
+            if (2 * kc > start && kc <= 4 * start) out.push_back({c, kc});
     return out;
 }
 
@@ -552,7 +555,7 @@ int r3d_batch_autotune(r3d_batch* b, const char* cache_path, int* rows_out, int*
     float best = 1e30f;
     int bcfg = kTileCfg, bkc = kTileChunk;
     if (b->n_tiled > 0)
-        for (auto [cfg, kc] : tile_candidates()) {
+        for (auto [cfg, kc] : tile_candidates(kTileChunk)) {
             b->tile_cfg = cfg;
             b->tile_kc = kc;
             const float ms = time_now();
@@ -659,12 +662,16 @@ int r3d_autotune(r3d_handle* h, const char* cache_path, int* cfg_out, int* kc_ou
     // again, longer and interleaved, so that run-to-run noise of a few per
     // cent does not pick a slower configuration
     std::vector<std::tuple<float, int, int>> seen[2];
-    for (auto [cfg, kc] : tile_candidates()) {
-        for (int kind = 0; kind < 2 && !rc; ++kind) {
+    for (int kind = 0; kind < 2 && !rc; ++kind) {
+        int dcfg = 0, dkc = 0;
+        tile_default(h->L, h->sms, kind != 0, &dcfg, &dkc);
+        auto cand = tile_candidates(dkc);
+        if (std::find(cand.begin(), cand.end(), std::make_pair(dcfg, dkc)) == cand.end()) cand.push_back({dcfg, dkc});
+        for (auto [cfg, kc] : cand) {
             const float ms = time_stage(cfg, kc, kind, 5);
             if (ms >= 0.f) seen[kind].emplace_back(ms, cfg, kc);
+            if (rc) break;
         }
-        if (rc) break;
     }
     float best[2] = {1e30f, 1e30f};
     int bc[2] = {c0, cr0}, bk[2] = {k0, kr0};

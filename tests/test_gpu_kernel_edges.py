@@ -221,6 +221,25 @@ def test_default_tiles(dims):
     assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
 
 
+@pytest.mark.parametrize("dims", [(47, 45, 43), (161, 133, 119), (255, 130, 131)])
+def test_autotune_sweep_size(dims):
+    """A sweep launches 24 stages for each of at most 7 z chunks of a
+    configuration and for the default, and times the three best of a kind three
+    times again (22 launches each), whatever the grid's size; the choice comes
+    from the candidates or is the default."""
+    chunks = set(r3d.tile_chunks())
+    with instance(dims) as ls:
+        ls.init_spheres_tg([(0.5, 0.5, 0.5, 0.25)], [(1, 0.5), (2, 0.3)])
+        default = ls.get_option(r3d.OPT_CHUNK), ls.get_option(r3d.OPT_CHUNK_REINIT)
+        before = ls.launch_count()
+        ls.autotune()
+        most = 2 * 12 * (7 * len(r3d.tile_configs()) + 1) + 2 * 3 * 3 * 22 + 8
+        assert 0 < ls.launch_count() - before <= most
+        for option, first in zip((r3d.OPT_CHUNK, r3d.OPT_CHUNK_REINIT), default):
+            kc = ls.get_option(option)
+            assert kc == first or (kc in chunks and first < 2 * kc and kc <= 4 * first)
+
+
 @pytest.mark.parametrize("precision", [r3d.FP32, r3d.FP64])
 @pytest.mark.parametrize("dims", [(40, 24, 18), (48, 1, 37)])
 @pytest.mark.parametrize("airy", [False, True])
