@@ -134,15 +134,26 @@ struct Scratch {
 // the step writes (fields, velocities, partials, scalars) is read by plain loads
 // through pointers without __restrict__: __ldg or a restricted parameter says
 // that it stays unwritten for the kernel's whole life, and lets the load move
-// above the wait.  step_next() allows the successor to be launched.  For grids of one wave (the successor finds room
-// beside them): a 2D flume of 600 x 75 cells stepped one call at a time
-// 1.64 -> 1.37 ms for ten steps, 128 x 128 in a graph 3.08 -> 2.92 ms for 60;
-// with several waves the wait of every block costs more than it hides (256^3
-// FP64 36.2 -> 37.4 ms for four steps), so larger grids run kernels without
-// it; nor did the tiled kernels gain, whose blocks fill the shared memory.
+// above the wait.  step_next() allows the successor to be launched.
+//
+// Where: grids of at most kStepBlocks blocks, whatever a block's size.  Measured
+// with and without, us a step of nine stages and three small kernels:
+//   steps called one by one, FP64 3D   592 blocks 84 / 82, 888 84 / 99, 1184
+//     105 / 130, 4000 248 / 270; 600 x 75 flume, ten steps, 1.37 / 1.64 ms
+//   in a graph, FP64 3D   144 57 / 57, 512 77 / 67, 888 82 / 83, 1184 106 / 106,
+//     4000 250 / 250; FP64 2D 144 44 / 46, 512 59 / 55, 888 67 / 67, 1184 88 / 89
+//   in a graph, FP32 2D   144 32 / 36, 512 34 / 38, 1184 40 / 42; stretched 3D
+//     144 44 / 48, 512 51 / 53, 888 62 / 55, 1184 63 / 62
+// So it gains where the host launches and on the smallest grids, and costs up
+// to 15 % in a graph at a few blocks per SM, whose early blocks crowd the SMs
+// that drain first; four steps of 256^3 FP64, of many waves, took 36.2 ms
+// without and 37.4 with (older kernels).  The line
+// is where a step called by itself still gains a fifth and a graph loses
+// nothing.  The tiled kernels, whose blocks fill the shared memory, gained
+// nowhere.
 __device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void step_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-constexpr long long kStepBlocks = 1184;  // of 128 threads and 64 registers on 148 SMs
+constexpr long long kStepBlocks = 1184;  // 8 per SM of 148
 inline bool step_grid(bool pdl, dim3 g) { return pdl && (long long)g.x * g.y * g.z <= kStepBlocks; }
 
 template <typename... P, typename... A>

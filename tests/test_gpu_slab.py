@@ -127,6 +127,34 @@ def test_native_domain_equals_undivided_grid(dims, nslabs, precision):
     assert np.array_equal(got[m], whole[r3d.PHI][m])
 
 
+@pytest.mark.parametrize("dims", [(32, 32, 37), (32, 32, 148), (32, 32, 149), (256, 1, 592), (256, 1, 596)])
+@pytest.mark.parametrize("precision", [r3d.FP64, r3d.FP32])
+@pytest.mark.parametrize("graph", [False, True])
+def test_early_launches_change_nothing(dims, precision, graph):
+    """An instance's kernels start while their predecessors drain up to 1184
+    blocks of 32 x 4 cells; a domain's slabs are launched plainly.  Steps with
+    the fluid update on grids either side of the line agree bit for bit, called
+    one by one and replayed, on a stretched grid (one cell per thread in both
+    forms)."""
+    from reef3d_b200.slab import Domain
+    nx, ny, nz = dims
+    xn, yn, zn, phi, vel = random_state(nx, ny, nz, seed=nz)
+    xn = xn + 0.1 * xn * (1.0 - xn / xn[-1])
+    out = []
+    for make in (lambda: r3d.LevelSet(nx, ny, nz, xn, yn, zn, precision=precision, **FLAGS),
+                 lambda: Domain(nx, ny, nz, xn, yn, zn, nslabs=2, precision=precision, devices=[0, 0], **FLAGS)):
+        with make() as d:
+            d.set_fluid(998.2, 1.004e-6, 1.205, 1.41e-5)
+            for f, a in zip((r3d.PHI, r3d.U, r3d.V, r3d.W), (phi, *vel)):
+                d.upload(f, a)
+            for _ in range(1 if graph else 6):
+                d.run(6 if graph else 1)
+            out.append([d.download(f) for f in (r3d.PHI, r3d.RO, r3d.VISC)])
+    m = visible_mask(*dims)
+    for a, b in zip(*out):
+        assert np.array_equal(a[m], b[m])
+
+
 @pytest.mark.parametrize("precision", [r3d.FP64, r3d.FP32])
 def test_native_domain_reconfigured_between_runs(precision):
     """Settings changed on the slabs after the domain's step graph was
