@@ -66,7 +66,7 @@ size_t footprint(const r3d_grid_desc* d, const Layout& L) {
     size_t b = 7 * (size_t)L.ncell * e;
     size_t tab = 0;
     const int n[3] = {d->nx, d->ny, d->nz};
-    for (int a = 0; a < 3; ++a) tab += 4 * (size_t)(n[a] + 21) + 2 * (size_t)(n[a] + 8) * 36 + 8;
+    for (int a = 0; a < 3; ++a) tab += 4 * (size_t)(n[a] + 21) + (size_t)(n[a] + 8) * 36 + 8;
     b += tab * (8 + 4);
     const long long blocks = (long long)((d->nx + 31) / 32) * ((d->ny + 3) / 4 + 4) * (d->nz + 4);
     b += (size_t)(blocks + (long long)d->ny * d->nz + 64) * 16 + 256;
@@ -76,31 +76,14 @@ size_t footprint(const r3d_grid_desc* d, const Layout& L) {
 template <typename T>
 void fill_kgrid(r3d_handle* h, KGrid<T>& g, T* base, std::vector<T>& host) {
     g.L = h->L;
-    size_t off = 0;
     host.clear();
     for (int a = 0; a < 3; ++a) {
-        const size_t o_dxp = off;
+        g.dxp[a] = base + host.size();
         for (double v : h->M.dxp[a]) host.push_back((T)v);
-        off = host.size();
-        const size_t o_dxn = off;
+        g.dxn[a] = base + host.size();
         for (double v : h->M.dxn[a]) host.push_back((T)v);
-        off = host.size();
-        const size_t o_qf = off;
-        for (double v : h->M.qf[a]) host.push_back((T)v);
-        off = host.size();
-        const size_t o_cf = off;
-        for (double v : h->M.cf[a]) host.push_back((T)v);
-        off = host.size();
-        const size_t o_isf = off;
-        for (double v : h->M.isf[a]) host.push_back((T)v);
-        off = host.size();
-        g.dxp[a] = base + o_dxp;
-        g.dxn[a] = base + o_dxn;
-        g.qf[a] = base + o_qf;
-        g.cf[a] = base + o_cf;
-        g.isf[a] = base + o_isf;
     }
-    // packed forms read by the FP64 stencils, each 16-byte aligned
+    // packed forms the stencils read, each 16-byte aligned in FP64
     for (int a = 0; a < 3; ++a) {
         while (host.size() % 4) host.push_back((T)0);
         g.dpr[a] = base + host.size();
@@ -135,8 +118,7 @@ void fill_kgrid(r3d_handle* h, KGrid<T>& g, T* base, std::vector<T>& host) {
 size_t metric_count(const r3d_handle* h) {
     size_t c = 0;
     for (int a = 0; a < 3; ++a)
-        c += h->M.dxp[a].size() + h->M.dxn[a].size() + h->M.qf[a].size() + h->M.cf[a].size() + h->M.isf[a].size()
-             + 2 * h->M.dxp[a].size() + 6 * h->M.cf[a].size() + 8;  // packed pairs and records, padding
+        c += 3 * h->M.dxp[a].size() + h->M.dxn[a].size() + 6 * h->M.cf[a].size() + 8;  // pairs, records, padding
     return c;
 }
 

@@ -124,7 +124,7 @@ __device__ __forceinline__ float conv_L(const KGrid<float>& g, const float* f, c
             if (g.x45 == 6) return deriv_tables_df6(fv, hv, plus, g.dxp[a], g.wt[a], t);
             return deriv_tables_df(fv, hv, plus, g.dxp[a], g.wt[a], t, g.x45, g.df_thr);
         }
-        return UNIFORM ? f32::deriv_uniform<float>(fv, plus, g.rh[a], g.eps_u * g.h[a] * g.h[a])
+        return UNIFORM ? f32::deriv_uniform(fv, plus, g.rh[a], g.eps_u * g.h[a] * g.h[a])
                        : f32::deriv_tables(fv, plus, g.dpr[a], g.wt[a], t);
     };
     float l = 0.0f;

@@ -26,8 +26,6 @@
 #include "stencil_f32.cuh"
 #include "tile_host.h"
 
-
-
 namespace r3d {
 
 namespace {
@@ -245,7 +243,6 @@ struct TileCfg {
 };
 
 // The configurations the library is built with (id = position).
-#ifndef R3D_TILE_CFGS
 #define R3D_TILE_CFGS(X)        \
     X(0, 64, 8, 1, 16, 3)       \
     X(1, 64, 8, 2, 12, 4)       \
@@ -254,7 +251,6 @@ struct TileCfg {
     X(4, 128, 8, 2, 8, 2)       \
     X(5, 64, 8, 1, 10, 4)       \
     X(6, 32, 16, 2, 12, 5)
-#endif
 
 #define R3D_CFG_TYPE(id, tx, ty, ry, ring, minb) using Cfg##id = TileCfg<tx, ty, ry, ring, minb>;
 R3D_TILE_CFGS(R3D_CFG_TYPE)
@@ -1009,11 +1005,7 @@ void tile_default(const Layout& L, int sms, bool reini, int* cfg, int* kc) {
     auto padded = [&](int c) { return columns(c) * info(c).tx * info(c).ty; };
     const int first = reini ? 6 : 1, other = reini ? 1 : 3;
     *cfg = 100 * padded(other) < 97 * padded(first) ? other : first;
-    tile_default_chunk(columns(*cfg) * L.nz, sms, *cfg, reini, kc);
-}
-
-void tile_default_chunk(long long planes, int sms, int cfg, bool reini, int* kc) {
-    const double waves = (double)planes / ((double)sms * info(cfg).minb);  // of one-plane items
+    const double waves = (double)(columns(*cfg) * L.nz) / ((double)sms * info(*cfg).minb);  // of one-plane items
     const int want = (int)(waves / (reini ? 7.0 : 2.2) + 0.5);
     const int lo = reini ? 1 : 2, hi = reini ? 8 : 10;
     *kc = want < lo ? lo : want > hi ? hi : want;

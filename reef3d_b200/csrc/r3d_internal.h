@@ -42,18 +42,11 @@ constexpr int kIoSkipLo = 1, kIoSkipHi = 2, kIoEdge = 4, kHaloZLo = 8, kHaloZHi 
 
 Layout make_layout(int nx, int ny, int nz);
 
-// Per-axis metric and WENO table offsets inside one device buffer of
-// doubles (FP64) and one of floats (FP32).  Index t = cell index + 5, the
-// reference's 1D indexing (src/iterators1D.h:25-60).
-struct AxisTables {
-    long long dxp, dxn;          // n + 21 entries each
-    long long qf, cf, isf;       // (n+8)*12, (n+8)*6, (n+8)*18 entries
-};
-
+// Index t = cell index + 5, the reference's 1D indexing (src/iterators1D.h:25-60).
 struct HostMetrics {
     int n[3];
     std::vector<double> xn[3], xp[3], dxn[3], dxp[3];
-    std::vector<double> qf[3], cf[3], isf[3];
+    std::vector<double> qf[3], cf[3], isf[3];  // WENO node tables: 12, 6, 18 values an index
     double dxm_mean;   // src/grid.cpp:102-148
     double dym, dzm;   // DIVEMesh header spacings (first node spacing)
     double psi;        // src/ini_psi.cpp:33-37
@@ -79,9 +72,6 @@ struct KGrid {
     // Q0..Q5, C0..C2, S0..S8 (record 2t + side), 16-byte aligned
     const T* wt[3];
     const T* dxn[3];
-    const T* qf[3];
-    const T* cf[3];
-    const T* isf[3];
     double f43;
     int f49;
     double psi;

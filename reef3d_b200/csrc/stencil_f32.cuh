@@ -19,43 +19,40 @@ namespace r3d {
 namespace f32 {
 
 template <typename R>
-__device__ __forceinline__ R rcp(R x) { return R(1) / x; }
-template <>
-__device__ __forceinline__ float rcp<float>(float x) { return __frcp_rn(x); }
-template <typename R>
 __device__ __forceinline__ R rsqrt_r(R x) { return rsqrt(x); }
 template <>
 __device__ __forceinline__ float rsqrt_r<float>(float x) { return rsqrtf(x); }
 
-// WENO5-HJ derivative on a uniform grid from the undivided differences
-// d1..d5 of the upwind set; eps = 1e-6*h^2.  Returns h * derivative.
-template <typename R>
-__device__ __forceinline__ R weno5_uniform(bool plus, R d1, R d2, R d3, R d4, R d5, R eps) {
+// WENO5-HJ derivative on a uniform grid in FP64 (the interface band) from the
+// undivided differences d1..d5 of the upwind set; eps = 1e-6*h^2.  Returns
+// h * derivative.
+__device__ __forceinline__ double weno5_uniform(bool plus, double d1, double d2, double d3, double d4, double d5,
+                                                double eps) {
     // IS of the stencils (d3,d4,d5), (d2,d3,d4), (d1,d2,d3):
     // 10/3 a^2 + 11/3 ab + 4/3 b^2 with a, b the differences to the middle q
-    const R a1 = d3 - d4, b1 = d5 - d4;
-    const R a2 = d4 - d3, b2 = d2 - d3;
-    const R a3 = d3 - d2, b3 = d1 - d2;
-    const R k10 = R(10.0 / 3.0), k11 = R(11.0 / 3.0), k4 = R(4.0 / 3.0);
-    const R is1 = (k10 * a1 + k11 * b1) * a1 + k4 * b1 * b1;
-    const R is2 = (k4 * a2 + R(5.0 / 3.0) * b2) * a2 + k4 * b2 * b2;
-    const R is3 = (k10 * a3 + k11 * b3) * a3 + k4 * b3 * b3;
-    const R s1 = is1 + eps, s2 = is2 + eps, s3 = is3 + eps;
-    const R r1 = rcp(s1), r2 = rcp(s2), r3 = rcp(s3);
-    R c1, c2, c3;
-    if (!plus) { c1 = R(0.3); c2 = R(0.6); c3 = R(0.1); }
-    else { c1 = R(0.1); c2 = R(0.6); c3 = R(0.3); }
-    const R al1 = c1 * r1 * r1, al2 = c2 * r2 * r2, al3 = c3 * r3 * r3;
-    const R inv = rcp(al1 + al2 + al3);
-    R p1, p2, p3;
+    const double a1 = d3 - d4, b1 = d5 - d4;
+    const double a2 = d4 - d3, b2 = d2 - d3;
+    const double a3 = d3 - d2, b3 = d1 - d2;
+    const double k10 = 10.0 / 3.0, k11 = 11.0 / 3.0, k4 = 4.0 / 3.0;
+    const double is1 = (k10 * a1 + k11 * b1) * a1 + k4 * b1 * b1;
+    const double is2 = (k4 * a2 + (5.0 / 3.0) * b2) * a2 + k4 * b2 * b2;
+    const double is3 = (k10 * a3 + k11 * b3) * a3 + k4 * b3 * b3;
+    const double s1 = is1 + eps, s2 = is2 + eps, s3 = is3 + eps;
+    const double r1 = 1.0 / s1, r2 = 1.0 / s2, r3 = 1.0 / s3;
+    double c1, c2, c3;
+    if (!plus) { c1 = 0.3; c2 = 0.6; c3 = 0.1; }
+    else { c1 = 0.1; c2 = 0.6; c3 = 0.3; }
+    const double al1 = c1 * r1 * r1, al2 = c2 * r2 * r2, al3 = c3 * r3 * r3;
+    const double inv = 1.0 / (al1 + al2 + al3);
+    double p1, p2, p3;
     if (!plus) {
-        p1 = d4 + R(1.0 / 3.0) * a1 - R(1.0 / 6.0) * b1;
-        p2 = d3 + R(1.0 / 3.0) * a2 - R(1.0 / 6.0) * b2;
-        p3 = d2 + R(1.0 / 3.0) * b3 + R(11.0 / 6.0) * a3;
+        p1 = d4 + (1.0 / 3.0) * a1 - (1.0 / 6.0) * b1;
+        p2 = d3 + (1.0 / 3.0) * a2 - (1.0 / 6.0) * b2;
+        p3 = d2 + (1.0 / 3.0) * b3 + (11.0 / 6.0) * a3;
     } else {
-        p1 = d4 + R(11.0 / 6.0) * a1 + R(1.0 / 3.0) * b1;
-        p2 = d3 + R(1.0 / 3.0) * b2 - R(1.0 / 6.0) * a2;
-        p3 = d2 + R(1.0 / 3.0) * a3 - R(1.0 / 6.0) * b3;
+        p1 = d4 + (11.0 / 6.0) * a1 + (1.0 / 3.0) * b1;
+        p2 = d3 + (1.0 / 3.0) * b2 - (1.0 / 6.0) * a2;
+        p3 = d2 + (1.0 / 3.0) * a3 - (1.0 / 6.0) * b3;
     }
     return (al1 * p1 + al2 * p2 + al3 * p3) * inv;
 }
@@ -142,20 +139,16 @@ __device__ __forceinline__ float weno5_mirrored(float d1, float d2, float d3, fl
     return p2 + (n1 * (p1 - p2) + n3 * (p3 - p2)) * rcp_fast(n1 + n2 + n3);
 }
 
-// Derivative along an axis from the 7 values f[-3..3] around the cell.
-// Uniform: returns the derivative (already divided by h).
-template <typename R>
-__device__ __forceinline__ R deriv_uniform(const R* fv, bool plus, R rh, R eps) {
-    // fv[0..6] = f[-3..3]
+// Derivative along an axis of a uniform grid from the 7 values fv[0..6] =
+// f[-3..3] around the cell (already divided by h).
+__device__ __forceinline__ double deriv_uniform(const double* fv, bool plus, double rh, double eps) {
     if (!plus)
-        return rh * weno5_uniform<R>(false, fv[1] - fv[0], fv[2] - fv[1], fv[3] - fv[2], fv[4] - fv[3],
-                                     fv[5] - fv[4], eps);
-    return rh * weno5_uniform<R>(true, fv[2] - fv[1], fv[3] - fv[2], fv[4] - fv[3], fv[5] - fv[4],
-                                 fv[6] - fv[5], eps);
+        return rh * weno5_uniform(false, fv[1] - fv[0], fv[2] - fv[1], fv[3] - fv[2], fv[4] - fv[3], fv[5] - fv[4],
+                                  eps);
+    return rh * weno5_uniform(true, fv[2] - fv[1], fv[3] - fv[2], fv[4] - fv[3], fv[5] - fv[4], fv[6] - fv[5], eps);
 }
 
-template <>
-__device__ __forceinline__ float deriv_uniform<float>(const float* fv, bool plus, float rh, float eps) {
+__device__ __forceinline__ float deriv_uniform(const float* fv, bool plus, float rh, float eps) {
     float D[6];
 #pragma unroll
     for (int m = 0; m < 6; ++m) D[m] = fv[m + 1] - fv[m];
@@ -193,7 +186,7 @@ __device__ __forceinline__ R reini_rhs_uniform(const R* fx, const R* fy, const R
         // minus side, plus side, or neither; one evaluation for both sides
         const bool c1 = xmin * lsSig > R(0) && xplus * lsSig > -xmin * lsSig;
         const bool c2 = xplus * lsSig < R(0) && xmin * lsSig < -xplus * lsSig;
-        const R d = deriv_uniform<R>(f, c2, rh[a], eps * hh[a]);
+        const R d = deriv_uniform(f, c2, rh[a], eps * hh[a]);
         g[a] = c1 || c2 ? d : R(0);
     }
     const R dnorm = sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);

@@ -54,9 +54,8 @@ struct TiledMember {
 int tile_cfg_count();
 int tile_cfg_describe(int cfg, int* tx, int* ty, int* ry, int* ring, int* threads);
 // The configuration and z chunk an instance starts with, by its size and the
-// device's SM count; the chunk alone for `planes` one-plane items in all.
+// device's SM count.
 void tile_default(const Layout& L, int sms, bool reini, int* cfg, int* kc);
-void tile_default_chunk(long long planes, int sms, int cfg, bool reini, int* kc);
 // Encodes the 3D tensor map of a padded FP32 field for the (TX+8) x (TY+6) x 1
 // plane boxes configuration `cfg` loads.  Returns 0 on success.
 int encode_plane_map(const Layout& L, const float* base, int cfg, CUtensorMap* out, std::string* why);

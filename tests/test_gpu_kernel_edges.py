@@ -1,7 +1,9 @@
 """Stage kernels, run loop and host copies at the sizes and values where they
-switch paths: the dealing of interface-band cells, steep fields, the FP64
-weights outside their fast range, the default tiles, the CFL maxima shared by
-a run's steps, and pageable copies around the piece size."""
+switch paths: the dealing of interface-band cells, steep fields, spikes and
+spacings at the ends of the FP32 range, the FP32 operators' error, the FP64
+weights outside their fast range, the default tiles and the autotuner's
+candidates, the CFL maxima shared by a run's steps, the Airy generator at its
+limits, rejected launches, and pageable copies."""
 import numpy as np
 import pytest
 
@@ -24,13 +26,17 @@ def dense(ls):
 
 
 @pytest.mark.parametrize("f49", [1, 0])
-@pytest.mark.parametrize("cells", [1, 3, 10, 11, 20, 21, 32, 64])
-def test_band_cells_dealt_to_lanes(cells, f49):
-    """A sheet that crosses `cells` cells of every row of 64 (one axis per lane
-    up to twenty cells of a warp's rows, three beyond): the tiled kernels
-    against the one-cell-per-thread ones.  Both form the band in FP64, so a
-    cell differs by the rounding of the other cells' FP32 right-hand sides:
-    two pseudo-steps of dtau <= h, RHS errors of a few ulp of 1."""
+@pytest.mark.parametrize("cfg", [0, 1, 6])
+@pytest.mark.parametrize("cells", [1, 3, 5, 6, 10, 11, 15, 16, 20, 21, 32, 64])
+def test_band_cells_dealt_to_lanes(cells, cfg, f49):
+    """A sheet that crosses `cells` cells of every row of 64: a warp of a 64 x 8
+    tile with one row a thread (configuration 0) holds `cells` band cells of a
+    plane, with two rows (1) twice as many, and of a 32 x 16 tile with two rows
+    (6) up to four times as many.  They are dealt out in rounds of ten cells up
+    to twenty, of 32 beyond.  The tiled kernels against the one-cell-per-thread
+    ones.  Both form the band in FP64, so a cell differs by the rounding of the
+    other cells' FP32 right-hand sides: two pseudo-steps of dtau <= h, RHS
+    errors of a few ulp of 1."""
     n = 64
     x = (np.arange(n) + 0.5) / n
     rng = np.random.default_rng(cells)
@@ -42,6 +48,7 @@ def test_band_cells_dealt_to_lanes(cells, f49):
     for tiled in (1, 0):
         with instance((n, n, n), f49=f49) as ls:
             ls.set_option(r3d.OPT_TILED, tiled)
+            ls.set_option(r3d.OPT_TILE_CFG, cfg)
             ls.upload(r3d.PHI, phi, r3d.LAYOUT_DENSE)
             ls.ghost_fill()
             ls.reinit(1)
@@ -54,9 +61,10 @@ def test_band_cells_dealt_to_lanes(cells, f49):
 @pytest.mark.parametrize("scale", [1.0, 1e2, 1e4, 1e7])
 @pytest.mark.parametrize("tiled", [1, 0])
 def test_steep_fields_fp32(scale, tiled):
-    """Gradients up to 1e7: the FP32 weights against FP64's.  The operator is
-    compared relative to its largest value; the smoothness indicators' FP32
-    differences of phi carry |phi| 2^-24 / h against gradients of order 1."""
+    """Gradients up to 1e7, jumps included: the FP32 operator against FP64's on
+    the same FP32 values, relative to its largest value.  An axis's derivative
+    is off by some 8 roundings of the largest difference in its stencil, of
+    which the derivative itself, from the smooth side, may be a small part."""
     n = 32
     rng = np.random.default_rng(3)
     res = []
@@ -71,13 +79,12 @@ def test_steep_fields_fp32(scale, tiled):
             ls.init_spheres_tg([(0.5, 0.5, 0.5, 0.2)], [(1, 0.5), (2, 0.25)])
             ls.upload(r3d.PHI, phi, r3d.LAYOUT_DENSE)
             ls.ghost_fill()
-            ls.set_dt(1e-3)
+            ls.set_dt(1e4)  # phi + dt L is dt L
             ls.stage(r3d.STAGE_CONVECTION, 1)
             ls.sync()
             res.append(ls.download(r3d.WORK1, r3d.LAYOUT_DENSE))
     assert np.all(np.isfinite(res[1]))
-    # dt |u| / h of the differences' error: 1e-3 * 1 * 32 * 8 ulp, and phi's own rounding
-    assert relmax(res[1], res[0]) <= 1e-3 * n * 64 * EPS32 + 4 * EPS32
+    assert relmax(res[1], res[0]) <= 64 * EPS32
 
 
 @pytest.mark.parametrize("spike", [10.0, 1e3, 1e6, 1e9, 1e12, 1e16])
@@ -240,6 +247,30 @@ def test_autotune_sweep_size(dims):
             assert kc == first or (kc in chunks and first < 2 * kc and kc <= 4 * first)
 
 
+@pytest.mark.parametrize("dims", [(33, 17, 5), (64, 40, 24), (96, 96, 96)])
+def test_instance_and_batch_defaults(dims):
+    """An instance alone and a batch's member start with different tiles and
+    chunks: the same level set, volume sums in another order (of at most
+    dims cells, each half an ulp)."""
+    out = []
+    for batched in (False, True):
+        with instance(dims) as ls:
+            ls.init_spheres_tg([(0.5, 0.4, 0.6, 0.2), (0.3, 0.6, 0.3, 0.1)], [(1, 0.5), (2, -0.3)])
+            if batched:
+                with r3d.Batch() as b:
+                    b.add(ls)
+                    b.step(3)
+                    b.sync()
+                    out.append((dense(ls), ls.last_volume()))
+            else:
+                ls.run(3)
+                ls.sync()
+                out.append((dense(ls), ls.last_volume()))
+    assert np.array_equal(out[0][0], out[1][0])
+    for x, y in zip(out[0][1], out[1][1]):
+        assert abs(x - y) <= 2.0 ** -53 * np.prod(dims) * abs(y)
+
+
 @pytest.mark.parametrize("precision", [r3d.FP32, r3d.FP64])
 @pytest.mark.parametrize("dims", [(40, 24, 18), (48, 1, 37)])
 @pytest.mark.parametrize("airy", [False, True])
@@ -279,9 +310,8 @@ def test_run_shares_cfl_maxima(precision, dims, airy):
 @pytest.mark.parametrize("nz", [11, 12, 24, 61, 128])
 @pytest.mark.parametrize("precision", [r3d.FP64, r3d.FP32])
 def test_pageable_copies(nz, precision):
-    """Host arrays below, at and beyond the size from which pageable copies
-    are split (4 MiB, in 1 MiB pieces), against a pinned array in one copy;
-    nx ny chosen so that 11 and 12 planes lie either side of 4 MiB."""
+    """Copies between pageable host arrays of 4 to 47 MB and the device against
+    the same fields through a pinned array, in both layouts."""
     import torch
     nx, ny = 220, 208
     a = np.random.default_rng(nz).standard_normal((nz, ny, nx)).astype(np.float32).astype(np.float64)
