@@ -70,13 +70,14 @@ __device__ __forceinline__ float rcp_fast(float x) {  // 1 ulp
 // whatever the others are (an indicator that overflows has weight 0).  Four
 // approximate reciprocals and no branch on the side, where four rounded ones,
 // five quotients and both sides' code made a stretched 160 x 128 x 96 grid
-// wait for them (stages of 40 / 66 us -> 37 / 50 us).
-// The result is the middle reconstruction plus the weighted differences of the
-// others to it: the weights' few ulp then count against those differences alone
-// (p1 w1 + p2 w2 + p3 w3 carries the sum's and the reciprocal's on the whole
-// derivative), and a convection operator is 7.0e-8 to 7.6e-8 off the 64-bit one in
-// the 2-norm (uniform grids 5.8e-8 to 7.1e-8), where the form with rounded
-// reciprocals and quotients was 9.3e-8 to 1.0e-7 (8.0e-8 to 9.5e-8) off.
+// wait for them (stages of 40 / 66 us -> 37 / 48 us).
+// The result is q3 plus the middle reconstruction's distance from it and the
+// weighted distances of the others to the middle one: the weights' few ulp
+// count against those alone (p1 w1 + p2 w2 + p3 w3 carries the sum's and the
+// reciprocal's on the whole derivative), and a convection operator is 6.5e-8 to
+// 7.2e-8 off the 64-bit one in the 2-norm (uniform grids 5.5e-8 to 6.8e-8), where
+// the form with rounded reciprocals and quotients was 9.3e-8 to 1.0e-7 (8.0e-8 to
+// 9.5e-8) off.
 // MASKS: the weight of stencil (q3,q4,q5) / (q2,q3,q4) / (q1,q2,q3) is 0 where
 // zero1..zero3 (the X45 = 6 masked differences; at least one stays on), and
 // the unscaled c_r / s_r^2 leave the FP32 range (no finite result) where the
@@ -99,10 +100,10 @@ __device__ __forceinline__ float weno5_tables(const float* __restrict__ W, bool 
     const float s3 = (S[6] * dq12 - S[7] * dq23) * dq12 + S[8] * dq23 * dq23 + 1.0e-6f;
     float n1, n2, n3;
     if (MASKS) {
-        const float r1 = __frcp_rn(s1), r2 = __frcp_rn(s2), r3 = __frcp_rn(s3);
-        n1 = zero1 ? 0.0f : C[0] * r1 * r1;
-        n2 = zero2 ? 0.0f : C[1] * r2 * r2;
-        n3 = zero3 ? 0.0f : C[2] * r3 * r3;
+        const float u1 = __frcp_rn(s1), u2 = __frcp_rn(s2), u3 = __frcp_rn(s3);
+        n1 = zero1 ? 0.0f : C[0] * u1 * u1;
+        n2 = zero2 ? 0.0f : C[1] * u2 * u2;
+        n3 = zero3 ? 0.0f : C[2] * u3 * u3;
     } else {
         const float m = fminf(s1, fminf(s2, s3));
         const float u1 = m * rcp_fast(s1), u2 = m * rcp_fast(s2), u3 = m * rcp_fast(s3);
@@ -110,15 +111,15 @@ __device__ __forceinline__ float weno5_tables(const float* __restrict__ W, bool 
         n2 = C[1] * u2 * u2;
         n3 = C[2] * u3 * u3;
     }
-    const float t1 = Q[1] * (q5 - q4);
+    const float t1 = Q[1] * dq54;
     const float x2 = plus ? dq23 : -dq34, y2 = plus ? -dq34 : dq23;
     const float x3 = plus ? -dq23 : dq12, y3 = plus ? dq12 : -dq23;
     const float t3 = Q[5] * y3;
-    const float p1 = q4 + Q[0] * dq34 + (plus ? t1 : -t1);
-    const float p2 = q3 + Q[2] * x2 - Q[3] * y2;
-    const float p3 = q2 + Q[4] * x3 + (plus ? -t3 : t3);
-    if (MASKS) return (n1 * p1 + n2 * p2 + n3 * p3) * __frcp_rn(n1 + n2 + n3);
-    return p2 + (n1 * (p1 - p2) + n3 * (p3 - p2)) * rcp_fast(n1 + n2 + n3);
+    const float r1 = Q[0] * dq34 + (plus ? t1 : -t1);
+    const float r2 = Q[2] * x2 - Q[3] * y2;
+    const float r3 = Q[4] * x3 + (plus ? -t3 : t3);
+    if (MASKS) return (n1 * (q4 + r1) + n2 * (q3 + r2) + n3 * (q2 + r3)) * __frcp_rn(n1 + n2 + n3);
+    return q3 + (r2 + (n1 * (r1 - (dq34 + r2)) + n3 * (r3 + (dq23 - r2))) * rcp_fast(n1 + n2 + n3));
 }
 
 // The uniform form in FP32 from the upwind set d1..d5 (the plus side passes
@@ -133,10 +134,11 @@ __device__ __forceinline__ float weno5_mirrored(float d1, float d2, float d3, fl
     const float m = fminf(s1, fminf(s2, s3));
     const float u1 = m * rcp_fast(s1), u2 = m * rcp_fast(s2), u3 = m * rcp_fast(s3);
     const float n1 = 0.3f * u1 * u1, n2 = 0.6f * u2 * u2, n3 = 0.1f * u3 * u3;
-    const float p1 = d4 + (1.0f / 3.0f) * a1 - (1.0f / 6.0f) * b1;
-    const float p2 = d3 - (1.0f / 3.0f) * a1 - (1.0f / 6.0f) * b2;
-    const float p3 = d2 + (1.0f / 3.0f) * b3 - (11.0f / 6.0f) * b2;
-    return p2 + (n1 * (p1 - p2) + n3 * (p3 - p2)) * rcp_fast(n1 + n2 + n3);
+    // the reconstructions as d3 + m2 (the middle one) and differences to it
+    const float m2 = -(1.0f / 3.0f) * a1 - (1.0f / 6.0f) * b2;
+    const float e1 = -(2.0f / 3.0f) * a1 - (1.0f / 6.0f) * b1 - m2;
+    const float e3 = (1.0f / 3.0f) * b3 - (5.0f / 6.0f) * b2 - m2;
+    return d3 + (m2 + (n1 * e1 + n3 * e3) * rcp_fast(n1 + n2 + n3));
 }
 
 // Derivative along an axis of a uniform grid from the 7 values fv[0..6] =

@@ -156,11 +156,11 @@ def test_spacings_fp32(e, dims):
 def test_convection_error_fp32(dims, stretch, tiled, roundings):
     """The FP32 convection operator against FP64's on the same (FP32) values, by
     its 2-norm: the roundings on the way of a value's leading part (difference,
-    two of the reconstruction, the correction's sum, 1/h, three of the
-    velocity and its product, the axes' sum: 9; quotient, its reciprocal's and
-    two of the tables: 13), each 0.42 2^-24 rms for mantissas spread over a
-    binade, added in quadrature.  Weights add nothing of that order: they
-    multiply differences of reconstructions."""
+    the reconstruction's sums, 1/h, three of the velocity and its product, the
+    axes' sum: up to 9; the quotient, its reciprocal's and two of the tables
+    more: 13), each 0.42 2^-24 rms for mantissas spread over a binade, added in
+    quadrature.  Weights add nothing of that order: they multiply differences of
+    reconstructions."""
     rng = np.random.default_rng(dims[0])
     nodes = []
     for n in dims:
