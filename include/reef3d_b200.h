@@ -499,8 +499,9 @@ int r3d_volume_dense_noalloc(const double* phi, int nx, int ny, int nz, double d
 
 /* ---------------------------------------------------------------- batches
  * Many FP32 instances of uneven sizes (2D and 3D mixed) advanced together:
- * one persistent launch per RK stage over a packed tile list of all members,
- * the whole step captured in a CUDA graph.  The reference has no
+ * per RK stage one launch over the packed items of all members on the tiled
+ * kernels and one over those of the others, the whole step captured in a CUDA
+ * graph.  The reference has no
  * counterpart (it runs one grid per process, src/weno_nug_func.h:198-202);
  * each member's step is levelset_RK3::start (src/levelset_RK3.cpp:103-172)
  * with its own CFL time step (src/ietimestep.cpp:38-206), clock and volume.
@@ -521,7 +522,7 @@ int r3d_batch_size(const r3d_batch* b, int* n);
 int r3d_batch_set_config(r3d_batch* b, int rows, int ctas_per_sm);
 int r3d_batch_get_config(const r3d_batch* b, int* rows, int* ctas_per_sm);
 /* Members on the tiled kernels (3D uniform FP32): tile configuration (as
- * R3D_OPT_TILE_CFG) and z chunk of the batch's persistent launches. */
+ * R3D_OPT_TILE_CFG) and z chunk of the batch's launches, one CTA per item. */
 int r3d_batch_set_tile_config(r3d_batch* b, int cfg, int chunk);
 int r3d_batch_get_tile_config(const r3d_batch* b, int* cfg, int* chunk);
 /* Times the candidate configurations on the batch (state-preserving): tile
@@ -588,8 +589,7 @@ int r3d_domain_fluid_update(r3d_domain* d, double* volume1, double* volume2);
  * 2.1, f49 1).  Submitted jobs wait in arrival order until their device
  * footprint (r3d_footprint) fits the HBM budget; admitted jobs stay
  * resident and advance together between polls -- FP32 jobs as members of
- * one batch (one persistent launch per RK stage over all members, CUDA
- * graph), FP64 jobs each on its own instance -- and leave when done.  A
+ * one batch (r3d_batch_*: all members in the same launches, CUDA graph), FP64 jobs each on its own instance -- and leave when done.  A
  * job's results do not depend on which jobs shared its steps.
  *  r3d_serve_poll: admits what fits, then advances every active job by up
  *    to max_steps steps, stopping at the first job to finish (which is

@@ -608,8 +608,8 @@ def _bcheck(rc, b=None):
 
 
 class Batch:
-    """Many FP32 instances advanced together (one persistent launch per RK
-    stage over all members, the step replayed from a CUDA graph)."""
+    """Many FP32 instances advanced together (every member in the same
+    launches of an RK stage, the step replayed from a CUDA graph)."""
 
     def __init__(self):
         load_library()

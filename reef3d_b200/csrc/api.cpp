@@ -593,7 +593,8 @@ int r3d_ls_step(r3d_handle* h, double dt) {
 // velocities, which nothing changes during a run (r3d_ls_run's steps scale
 // them by the velocity factor alone; the Airy generator rewrites u and w and
 // finds their maxima on the way, so only v's stays).  Taken per step they
-// were 41 of 1450 us at 256^3 and three of thirteen launches.
+// were 41 of 1450 us at 256^3 and two launches and a clear of a small step's
+// thirteen.
 int enqueue_run_start(r3d_handle* h, int adaptive) {
     if (!adaptive) return R3D_OK;
     h->launches += launch_vmax(h->L, h->field[R3D_U], h->field[R3D_V], h->field[R3D_W], fp32(h), h->S, h->stream);

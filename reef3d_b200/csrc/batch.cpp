@@ -1,6 +1,6 @@
-// Batched execution of many FP32 instances: one persistent launch per RK
-// stage over a packed tile list of all members, the whole step captured in
-// a CUDA graph and replayed, the tile shape and grid size picked by an
+// Batched execution of many FP32 instances: per RK stage one launch over the
+// items of all tiled members (one CTA each) and, beside it, a persistent one over
+// the tiles of the others, the whole step captured in a CUDA graph and replayed, the tile shape and grid size picked by an
 // autotuner whose choice is cached per size class.
 #include <cuda_runtime.h>
 

@@ -1,5 +1,5 @@
-// Batched persistent kernels: many FP32 instances of uneven sizes, 2D and
-// 3D mixed, advanced together.  The work of a stage is a packed list of
+// Batched persistent kernels of the members that run one cell per thread (2D,
+// stretched), FP32 instances of uneven sizes advanced together.  The work of a stage is a packed list of
 // tiles (32 x ROWS cells: x by y rows of one z plane in 3D, x by z rows in
 // 2D) over all members; a persistent grid walks the list, each CTA looking
 // up its member by binary search over the members' first tile index.

@@ -1,9 +1,8 @@
 // Continuous-batching job server behind the C-ABI (r3d_serve_*): transport
 // jobs wait in arrival order until their device footprint fits the HBM
 // budget, every admitted job stays resident on the device, and all active
-// jobs advance together -- FP32 jobs as members of one batch (one persistent
-// launch per RK stage over every member, the step replayed from a CUDA
-// graph), FP64 jobs each on its own instance.  Jobs join and leave between
+// jobs advance together -- FP32 jobs as members of one batch (every member in
+// the same launches of an RK stage, the step replayed from a CUDA graph), FP64 jobs each on its own instance.  Jobs join and leave between
 // steps; a job's result does not depend on which others shared its steps.
 #include <cuda_runtime.h>
 

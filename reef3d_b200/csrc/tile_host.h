@@ -64,7 +64,8 @@ int launch_tile_stage(const CUtensorMap& map, const TileArgs& a, int cfg, bool r
 // Sets the tiled kernels' shared-memory attributes on the current device
 // (once per device); false when the device refuses them.
 bool tile_prepare();
-// CTAs per SM configuration `cfg` is built to co-reside (persistent grids)
+// CTAs per SM configuration `cfg` is built to co-reside (the persistent grid of
+// launch_batch_tile_vmax)
 int tile_ctas_per_sm(int cfg);
 long long tile_items_of(const Layout& L, int kc, int cfg);
 // Batched tiled stage over the `grid` items of nm tiled members, whose maps

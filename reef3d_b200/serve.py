@@ -5,8 +5,8 @@ given number of steps) arrive over time.  The native serving runtime
 (r3d_serve_*, reef3d_b200/csrc/serve.cpp) admits waiting jobs in arrival
 order whenever their device footprint fits the HBM budget, keeps every
 admitted job's fields resident on the device, and advances all active jobs
-together in one batch (one persistent launch per RK stage over every
-member, the step replayed from a CUDA graph).  Jobs join and leave between
+together in one batch (every member in the same launches of an RK stage,
+the step replayed from a CUDA graph).  Jobs join and leave between
 steps, so work of jobs that arrive while others are on the GPU overlaps
 with theirs on the device.  A job's result does not depend on which other
 jobs shared its steps.  ``TransportServer`` feeds it a timed job stream.

@@ -1,5 +1,5 @@
-"""Batched persistent execution (many FP32 instances, 2D and 3D mixed, one
-launch per RK stage, CUDA graph).  A member's result must not depend on the
+"""Batched execution (many FP32 instances, 2D and 3D mixed, in the same launches
+of an RK stage, CUDA graph).  A member's result must not depend on the
 batch around it: alone and in the mix it is bit-identical (same kernels,
 same per-member reductions); against the FP64 oracle it meets the FP32
 tolerance of test_gpu_fp32.py."""
