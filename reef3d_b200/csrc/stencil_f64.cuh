@@ -106,11 +106,13 @@ __device__ __noinline__ double weno5_any(const double* __restrict__ W, bool plus
 // Where the ends round apart, about one evaluation in 2^17, or one of A, B, C
 // (1e-12 and up by psi) leaves [2^-511, 2^499), compared on the high words,
 // weno5_any divides: all are the IEEE quotients.  At 256^3, us per stage 1 / 2:
-// convection 798 / 830 with six IEEE divisions, 709 / 741 so; reinitialisation
-// 838 / 882 and 791 / 840.  (One residual correction per quotient with the
+// convection 798 / 830 with six IEEE divisions, 714 / 752 so; reinitialisation
+// 838 / 882 and 792 / 828.  (One residual correction per quotient with the
 // product of two reciprocals, without the second end, took 778 / 747 and 813 /
 // 855, with more spilled registers, and was an ulp off where a quotient lies next
-// to the middle of two doubles.)
+// to the middle of two doubles.)  The reconstruction goes before the test of the
+// ends, whose chain it then covers: 60 steps of 128 x 128 2.60 -> 2.56 ms, of
+// 300 x 75 2.69 -> 2.61 ms (256^3 convection 705 / 736 the other way round).
 __device__ __forceinline__ double weno5(const double* __restrict__ W, bool plus, double q1, double q2, double q3,
                                         double q4, double q5) {
     double A, B, C;
@@ -127,8 +129,9 @@ __device__ __forceinline__ double weno5(const double* __restrict__ W, bool plus,
     const double w1 = bracket_div(c0, A * sum, yA * ys, apart);
     const double w2 = bracket_div(c1, B * sum, yB * ys, apart);
     const double w3 = bracket_div(c2, C * sum, yC * ys, apart);
-    if (apart) return weno5_any(W, plus, q1, q2, q3, q4, q5);
-    return reconstruct(W, plus, q1, q2, q3, q4, q5, w1, w2, w3);
+    double v = reconstruct(W, plus, q1, q2, q3, q4, q5, w1, w2, w3);
+    if (apart) v = weno5_any(W, plus, q1, q2, q3, q4, q5);
+    return v;
 }
 
 // Upwind-biased derivative along one axis (stride s) at linear index c,
