@@ -366,7 +366,7 @@ def test_airy_run_at_the_shared_memory_limits(edge, precision):
 
 def test_airy_refused_beyond_shared_memory():
     """One cell more than the tables' limit is refused when the generator is
-    set, as before it is used."""
+    set."""
     with pytest.raises(r3d.R3DError):
         airy_flume(14517 - 56, 56, r3d.FP32).close()
 
