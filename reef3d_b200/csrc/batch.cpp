@@ -51,10 +51,14 @@ struct r3d_batch {
     // tile configuration and z chunk of the tiled members' launches (the
     // batch encodes its own tensor maps of their fields for it)
     // The default does not look at the members: the order of a member's
-    // volume sums follows it and must not depend on the batch around it.  On
-    // 16 / 5 members of 64..160 / 45..112 cells an edge a step took 1.64 /
-    // 0.40 ms with it, 1.60 / 0.42 at best for the first, 1.73 / 0.38 at best
-    // for the second, 1.64 / 0.61 with configuration 0 and 16 planes before.
+    // volume sums follows it and must not depend on the batch around it.
+    // Measured, ms a step with it / with the best of seven configurations and
+    // chunks 4..16 / with configuration 0 and 16 planes: 3 members of 33..77
+    // cells an edge 0.30 / 0.18 / 0.39, 16 of 24..64 0.38 / 0.32 / 0.45, one of
+    // 128 0.30 / 0.27 / 0.41, 32 of 48..96 1.98 / 1.85 / 2.05, 4 of 112..160
+    // 1.02 / 1.02 / 1.13, 16 of 64..160 half of them 2D 1.57 / 1.49 / 1.67, 64 of
+    // 64..128 half 2D 3.89 / 3.68 / 3.98, 8 of 160..224 5.48 / 5.04 / 5.55, 2 of 256
+    // 2.71 / 2.53 / 2.67.  r3d_batch_autotune finds the difference.
     int tile_cfg = kTileCfg;
     bool tile_iso = false;  // every tiled member has cubic cells (tile_args_iso)
     int tile_kc = kTileChunk;
